@@ -57,6 +57,15 @@ struct DevParams {
     float vl_half_skin;  // lists stay valid while the displacement bound is below this
     uint32_t vl_cap;     // neighbours per bead list
     float ibox[3];       // 1 / box on periodic axes, 0 on the others (min_image_near)
+    // SRD grid: multiply-shift divisors by its x extent and its layer, cells
+    // per unit length (0 on axes of one cell), the box's middle and the
+    // distance from it up to which positions count as near the box, and whether
+    // every axis tiles the box (a step across the periodic boundary is then a
+    // step by one cell)
+    uint32_t sdiv_x_m, sdiv_x_k, sdiv_xy_m, sdiv_xy_k;
+    float srd_per_len[3], srd_mid[3], srd_reach[3];
+    int32_t srd_tiles_box;
+    int32_t srd_flat;  // one layer, both axes periodic
 };
 
 // Planar systems (two-dimensional WCA worms) compute with two vector

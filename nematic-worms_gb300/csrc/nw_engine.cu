@@ -97,6 +97,18 @@ DevParams make_dev_params(const NwConfig& c, float dt)
         }
         P.lncells *= P.lgrid[a];
     }
+    fast_div_params(P.srd_grid[0], P.sdiv_x_m, P.sdiv_x_k);
+    fast_div_params(P.srd_grid[0] * P.srd_grid[1], P.sdiv_xy_m, P.sdiv_xy_k);
+    P.srd_flat = P.srd_grid[2] == 1u && P.bnd[0] == NW_PERIODIC && P.bnd[1] == NW_PERIODIC &&
+                 P.srd_grid[0] < (1u << 24) && P.srd_grid[1] < (1u << 24);  // 24-bit products of the mask hash
+    P.srd_tiles_box = 1;
+    for (int a = 0; a < 3; ++a) {
+        P.srd_per_len[a] = P.srd_grid[a] > 1u ? P.srd_inv_cell[a] : 0.0f;
+        P.srd_mid[a] = P.origin[a] + 0.5f * P.box[a];
+        P.srd_reach[a] = P.srd_grid[a] > 1u ? P.box[a] : INFINITY;
+        const double tiled = (double)P.srd_grid[a] * P.srd_cell[a];
+        if (P.srd_grid[a] > 1u && !(std::fabs(tiled - P.box[a]) <= 1e-6 * P.box[a])) P.srd_tiles_box = 0;
+    }
     fast_div_params(P.lgrid[0], P.ldiv_x_m, P.ldiv_x_k);
     fast_div_params(P.lgrid[0] * P.lgrid[1], P.ldiv_xy_m, P.ldiv_xy_k);
     return P;
@@ -146,7 +158,7 @@ uint64_t enqueue_bead_step(const DevParams& P, const StepBuffers& B, uint32_t nc
     chunk_sum_kernel<<<nchunks, 512, 0, s>>>(B.cell_count, P.ncells, B.chunk_count, nullptr, nullptr);
     NW_MARK("scan_cells");
     scan_cells_kernel<true><<<nchunks, 512, 0, s>>>(B.cell_count, B.chunk_count, P.ncells, B.cell_offset, B.cell_start,
-                                                    B.cell_end, nullptr, nullptr, nullptr);
+                                                    B.cell_end, nullptr, nullptr, nullptr, nullptr, nullptr);
     NW_MARK("scatter");
     scatter_kernel<<<cdiv(P.nb, 256), 256, 0, s>>>(B.hash, B.slot, B.cell_offset, B.tmp_index, P.nb);
     if (P.model == NW_MODEL_REF_DEM) {
@@ -166,30 +178,6 @@ uint64_t enqueue_bead_step(const DevParams& P, const StepBuffers& B, uint32_t nc
         pair_wca_kernel<<<cdiv(P.nb, 256), 256, 0, s>>>(P, B);
     }
     return 6;
-}
-
-uint64_t enqueue_srd(const DevParams& P, const StepBuffers& B, uint32_t srd_nchunks, uint32_t step_off, float dt_srd,
-                     int shift_from_step, float3 shift, cudaStream_t s, Prof* prof, uint32_t buf_sel)
-{
-    if (P.ntotal == 0) return 0;
-    NW_MARK("srd_hash");
-    srd_hash_kernel<<<cdiv(P.ntotal, 256), 256, 0, s>>>(P, B, step_off, shift_from_step, shift, buf_sel);
-    NW_MARK("srd_chunk_sum");
-    // bead and solvent counts side by side (grid rows 0 and 1)
-    chunk_sum_kernel<<<dim3(srd_nchunks, 2), 512, 0, s>>>(B.srd_bcount, P.srd_ncells, B.srd_bchunk, B.srd_scount,
-                                                          B.srd_schunk);
-    NW_MARK("srd_scan_cells");
-    scan_cells_kernel<false><<<dim3(srd_nchunks, 2), 512, 0, s>>>(B.srd_bcount, B.srd_bchunk, P.srd_ncells,
-                                                                  B.srd_boff, nullptr, nullptr, B.srd_scount,
-                                                                  B.srd_schunk, B.srd_soff);
-    NW_MARK("srd_scatter");
-    srd_scatter_kernel<<<cdiv(P.ntotal, 256), 256, 0, s>>>(P, B);
-    NW_MARK("srd_collide");
-    srd_collide_kernel<<<cdiv(P.srd_ncells, 128), 128, 0, s>>>(P, B, step_off, dt_srd, buf_sel);
-    NW_MARK("srd_collide_big");
-    srd_collide_big_kernel<<<kSrdBigBlocks, kBigWarps * 32, 0, s>>>(P, B, step_off, dt_srd, buf_sel);
-    srd_flip_kernel<<<1, 1, 0, s>>>(B.scur);
-    return 7;
 }
 
 // Histogram of bead hashes (the counting sort's first pass, for the sorted
@@ -468,12 +456,25 @@ cudaError_t ensure_sorted(nw_system* s)
     count_hash_kernel<<<cdiv(s->nb, 256), 256, 0, s->stream>>>(B.hash, s->nb, B.cell_count, B.slot);
     chunk_sum_kernel<<<s->nchunks, 512, 0, s->stream>>>(B.cell_count, P.ncells, B.chunk_count, nullptr, nullptr);
     scan_cells_kernel<true><<<s->nchunks, 512, 0, s->stream>>>(B.cell_count, B.chunk_count, P.ncells, B.cell_offset,
-                                                               B.cell_start, B.cell_end, nullptr, nullptr, nullptr);
+                                                               B.cell_start, B.cell_end, nullptr, nullptr, nullptr, nullptr,
+                                                               nullptr);
     scatter_kernel<<<cdiv(s->nb, 256), 256, 0, s->stream>>>(B.hash, B.slot, B.cell_offset, B.tmp_index, s->nb);
     stable_gather_kernel<false><<<cdiv(s->nb, 256), 256, 0, s->stream>>>(P, B);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) s->sorted_for = s->step;
     return e;
+}
+
+// The stored solvent no longer lies in its cells' order (positions set from
+// outside, or another grid): the next collision buckets it.
+cudaError_t release_solvent_order(nw_system* s)
+{
+    if (!s->B.srd_state) return cudaSuccess;
+    for (int k = 0; k < 2; ++k) {
+        const cudaError_t e = cudaMemsetAsync(s->B.srd_state + kSrdGeo + 8 * k + kSrdHeld, 0, 4, s->stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 enum class Dir { ToDevice, ToHost };
@@ -575,6 +576,7 @@ nw_status transfer(nw_system* s, int array, void* host, uint32_t start, uint32_t
         char* d = static_cast<char*>(solv_ptr) + (a - nbead) * elem;
         e = dir == Dir::ToDevice ? cudaMemcpyAsync(d, h, (b - a) * elem, cudaMemcpyHostToDevice, s->stream)
                                  : cudaMemcpyAsync(h, d, (b - a) * elem, cudaMemcpyDeviceToHost, cs);
+        if (e == cudaSuccess && dir == Dir::ToDevice && array == NW_POSITION) e = release_solvent_order(s);
     }
     if (e == cudaSuccess && early) {
         e = cudaEventRecord(s->aux_done, s->aux);
@@ -713,7 +715,11 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         A(alloc_n(s, &B.srd_bcount, Cs + 8));
         A(alloc_n(s, &B.srd_scount, Cs + 8));
         A(alloc_n(s, &B.srd_boff, Cs + 8));
-        A(alloc_n(s, &B.srd_soff, Cs + 8));
+        for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.srd_soff2[k], Cs + 8));
+        A(alloc_n(s, &B.srd_btab, Cs * 4));
+        A(alloc_n(s, &B.srd_bhead, Cs));
+        A(alloc_n(s, &B.srd_bnext, nb));
+        A(alloc_n(s, &B.srd_state, kSrdWords));
         A(alloc_n(s, &B.srd_start, Cs + 8));
         A(alloc_n(s, &B.srd_end, Cs + 8));
         A(alloc_n(s, &B.srd_bchunk, (size_t)s->srd_nchunks + 1));
@@ -757,6 +763,8 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         Z(B.srd_bcount, ((size_t)s->srd_ncells + 8) * 4);
         Z(B.srd_scount, ((size_t)s->srd_ncells + 8) * 4);
         Z(B.srd_mean, (size_t)s->srd_ncells * 16);
+        Z(B.srd_bhead, (size_t)s->srd_ncells * 4, 0xff);
+        Z(B.srd_state, kSrdWords * 4);
     }
     Z(B.err, 16);
     Z(B.step_base, 8);
@@ -805,7 +813,7 @@ nw_status nw_set_config(nw_system* s, const NwConfig* cfg)
     s->hash_for = ~0ull;
     s->sorted_for = ~0ull;
     drop_graphs(s);
-    return NW_OK;
+    return cuda_status(release_solvent_order(s));  // the box or the cells may have changed
 }
 
 nw_status nw_get_config(const nw_system* s, NwConfig* cfg)

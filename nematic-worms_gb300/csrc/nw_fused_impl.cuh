@@ -19,8 +19,6 @@
 // order as with the sorted arrays, and runs are bit-identical.
 #pragma once
 
-#include <utility>
-
 #include "nw_fused.cuh"
 
 namespace nw {
@@ -36,45 +34,6 @@ __device__ __forceinline__ T* pick2(T* const (&a)[2], uint32_t k)
 __device__ __forceinline__ uint32_t* pick3(uint32_t* const (&a)[3], uint32_t k)
 {
     return k == 0u ? a[0] : (k == 1u ? a[1] : a[2]);
-}
-
-// Programmatic dependent launch: the step kernels are launched with the
-// stream-serialisation attribute relaxed, so that a kernel's blocks may be
-// scheduled while the previous kernel's last blocks still run.  Each step
-// kernel first waits (griddepcontrol.wait) until the previous kernel has
-// completed and its writes are visible, exactly the stream order, and then
-// lets the next launch begin.  Launched without the attribute both
-// instructions return at once.  NW_PDL=0 builds plain launches.
-#ifndef NW_PDL
-#define NW_PDL 1
-#endif
-__device__ __forceinline__ void pdl_enter()
-{
-#if NW_PDL
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
-
-template <class... KArgs, class... Args>
-inline void launch_pdl(void (*kernel)(KArgs...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s,
-                       Args&&... args)
-{
-#if NW_PDL
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-#else
-    kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
-#endif
 }
 
 // Ascending bitonic sort of N (power of two) registers, fully unrolled.

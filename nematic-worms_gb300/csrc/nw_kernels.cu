@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(512) chunk_sum_kernel(const uint32_t* __restri
                                                         uint32_t* __restrict__ chunk, const uint32_t* __restrict__ a2,
                                                         uint32_t* __restrict__ chunk2)
 {
+    pdl_enter();
     if (blockIdx.y) {
         a = a2;
         chunk = chunk2;
@@ -464,448 +465,6 @@ __global__ void __launch_bounds__(256) pair_wca_kernel(const DevParams P, const 
     if (planar_system(P)) pair_wca<2>(P, S);
     else pair_wca<3>(P, S);
 }
-
-// SRD cell hash of every particle (beads from the current bead buffer,
-// solvent from the current solvent buffer) and its slot in its cell's bead
-// or solvent bucket.  The solvent is stored in cell order, so equal keys come
-// in runs along the warp: the first lane of each run takes the run's slots
-// with one atomic.  The grid shift of a scheduled collision is drawn once per
-// block.
-__global__ void __launch_bounds__(256) srd_hash_kernel(const DevParams P, const StepBuffers S, uint32_t step_off,
-                                                       int shift_from_step, float3 shift, uint32_t buf_sel)
-{
-    __shared__ float s_shift[3];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < P.ntotal;
-    const bool bead = i < P.nb;
-    // the step counter and the solvent buffer index side by side, then the
-    // particle's position, all before the shift's barrier
-    const unsigned long long step = *S.step_base + step_off;
-    const uint32_t sc = *S.scur;
-    const uint32_t cur = buf_sel < 2u ? buf_sel : (uint32_t)(step & 1ull);
-    float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) p4 = bead ? S.pos2[cur][i] : S.spos2[sc][i - P.nb];
-    if (shift_from_step) {
-        if (threadIdx.x == 0) {
-            const float3 d = srd_shift_of(P, step);
-            s_shift[0] = d.x;
-            s_shift[1] = d.y;
-            s_shift[2] = d.z;
-        }
-        __syncthreads();
-        shift = make_float3(s_shift[0], s_shift[1], s_shift[2]);
-    }
-    uint32_t h = 0, key = 0xffffffffu;  // no cell hash reaches 2^31 - 1 with the bead bit set
-    if (valid) {
-        h = srd_hash(P, f3(p4), shift);
-        S.srd_hash[i] = h;
-        key = h | (bead ? 0x80000000u : 0u);
-    }
-    // every lane of the warp takes part (blockDim is a multiple of 32)
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0u || prev != key);
-    const uint32_t upto = (2u << lane) - 1u;  // lanes 0..lane (all 32 bits for lane 31)
-    const uint32_t start = 31u - (uint32_t)__clz(heads & upto);
-    const uint32_t after = heads & ~upto;
-    const uint32_t end = after ? (uint32_t)(__ffs(after) - 1) : 32u;
-    uint32_t base = 0;
-    if (valid && lane == start) base = atomicAdd(bead ? &S.srd_bcount[h] : &S.srd_scount[h], end - start);
-    base = __shfl_sync(0xffffffffu, base, (int)start);
-    if (valid) S.srd_slot[i] = base + (lane - start);
-}
-
-// Bucket every particle: beads by bead index, solvent by solvent index.
-__global__ void __launch_bounds__(256) srd_scatter_kernel(const DevParams P, const StepBuffers S)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.ntotal) return;
-    if (i == 0) *S.srd_nbig = 0;  // the list is filled by the collision that follows
-    const uint32_t h = S.srd_hash[i], slot = S.srd_slot[i];
-    if (i < P.nb) S.srd_btmp[S.srd_boff[h] + slot] = i;
-    else S.srd_stmp[S.srd_soff[h] + slot] = i - P.nb;
-}
-
-// SRD collision.  A warp owns 32 consecutive cells; their members are one
-// contiguous range of the stable (cell, index) order and their solvent one
-// contiguous range of the new solvent storage.  So the warp gathers the
-// members' velocities and positions lane-strided into shared memory (the
-// previous collision's cell order keeps them in a compact region), each
-// thread takes its own cell's sums from shared memory, every lane then
-// updates the members of its slots, and the warp writes the stable order and
-// the streamed solvent back coalesced.
-//
-// Per cell, in the member order (the cell's beads, then its solvent, each by
-// index): the reference's isokinetic scaling (particles_kernel_impl.cuh:605-637)
-// or none, the mass-weighted cell mean (:560-594), the +/- alpha rotation of
-// (v - u) (:640-691), the relative-velocity thermostat when selected, and the
-// solvent's ballistic streaming by dt_srd (solvent_integrator, :145-205).
-// Beads are written in place, the solvent to the other solvent buffer.
-// A warp holding more than kWarpCap members takes its cells in rounds that
-// fit.  A cell of more than kLaneCap members goes to srd_collide_big_kernel
-// (a warp per cell), so that no lane's serial loops run far longer than its
-// neighbours'.
-constexpr int kCollideWarps = 4;
-// 192 members per warp (32 cells at up to 6 members on average) keeps
-// 8 blocks of 4 warps resident per SM (27 KB of shared memory, 64 registers).
-constexpr uint32_t kWarpCap = 192;
-static_assert(kLaneCap <= kWarpCap, "a cell of the warp path fits the staging alone");
-static_assert(5 * ((kWarpCap + 31) / 32) <= 32, "a lane's slot-to-cell fields fit one register");
-
-__global__ void __launch_bounds__(kCollideWarps * 32, 8) srd_collide_kernel(const DevParams P, const StepBuffers S,
-                                                                         uint32_t step_off, float dt_srd,
-                                                                         uint32_t buf_sel)
-{
-    __shared__ uint32_t s_id[kCollideWarps][kWarpCap];
-    __shared__ float4 s_v[kCollideWarps][kWarpCap];
-    __shared__ float4 s_p[kCollideWarps][kWarpCap];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = c < P.srd_ncells;
-    const unsigned long long step = *S.step_base + step_off;
-    const uint32_t cur = buf_sel < 2u ? buf_sel : (uint32_t)(step & 1ull);
-    const uint32_t a = *S.scur;
-    const float4* __restrict__ sv_old = S.svel2[a];
-    const float4* __restrict__ sp_old = S.spos2[a];
-    float4* __restrict__ sv_new = S.svel2[a ^ 1u];
-    float4* __restrict__ sp_new = S.spos2[a ^ 1u];
-    float4* __restrict__ bvel = S.vel2[cur];
-    uint32_t b0 = 0, nbc = 0, s0 = 0, nsc = 0;
-    if (valid) {
-        b0 = S.srd_boff[c];
-        nbc = S.srd_boff[c + 1] - b0;
-        s0 = S.srd_soff[c];
-        nsc = S.srd_soff[c + 1] - s0;
-    }
-    const uint32_t nall = nbc + nsc;
-    const uint32_t start = b0 + s0;  // particles before this cell in the stable order
-    if (valid) {
-        S.srd_start[c] = nall ? start : kEmpty;
-        S.srd_end[c] = nall ? start + nall : kEmpty;
-    }
-    // a cell of more than kLaneCap members is collided by a whole warp in
-    // srd_collide_big_kernel; here it counts as empty
-    const bool big = nall > kLaneCap;
-    if (valid && big) S.srd_big[atomicAdd(S.srd_nbig, 1u)] = c;
-    const uint32_t n = big ? 0u : nall;
-    const uint32_t incl = warp_incl_scan(n);
-    const uint32_t loc = incl - n;  // this cell's members in the warp's staging
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0u) {  // uniform over the warp
-        if (valid && !big) S.srd_mean[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
-    }
-    const uint32_t gdelta = start - loc;  // stable-order position of staged slot j of this cell: gdelta + j
-    // Rounds of consecutive cells whose members fit the staging buffers
-    // (one round unless the warp holds more than kWarpCap members).
-    uint32_t first = 0;
-    while (first < 32u) {
-        const uint32_t base = __shfl_sync(0xffffffffu, loc, (int)first);
-        const uint32_t fm = __ballot_sync(0xffffffffu, lane >= first && loc + n - base <= kWarpCap);
-        const uint32_t last = 31u - (uint32_t)__clz(fm);
-        const uint32_t rtotal = __shfl_sync(0xffffffffu, loc + n, (int)last) - base;
-        const bool mine = lane >= first && lane <= last;
-        // members of the round's cells in stable order: ids < nb are beads, nb + k
-        // is solvent k.  The bucket entries are loaded lane-strided (consecutive
-        // cells' entries are consecutive in the buckets), each into its cell's
-        // segment; then every lane orders its own cell's segment in shared memory.
-        // A lane visits the same slots (j0 + lane) in the three loops below, so
-        // the cell of each of its (at most kWarpCap / 32 = 6) slots is found once
-        // and kept in 5-bit fields of one register.
-        uint32_t qpack = 0;
-#pragma unroll 2
-        for (uint32_t j0 = 0; j0 < rtotal; j0 += 32u) {
-            const uint32_t j = j0 + lane, slot = base + (j < rtotal ? j : 0u);
-            uint32_t q = 0;  // the last cell whose segment starts at or before slot
-#pragma unroll
-            for (uint32_t st = 16; st; st >>= 1) {
-                const uint32_t lq = __shfl_sync(0xffffffffu, loc, (int)(q + st));
-                if (lq <= slot) q += st;
-            }
-            qpack |= q << (5u * (j0 >> 5));
-            const uint32_t lq = __shfl_sync(0xffffffffu, loc, (int)q), nq = __shfl_sync(0xffffffffu, nbc, (int)q);
-            const uint32_t bq = __shfl_sync(0xffffffffu, b0, (int)q), sq = __shfl_sync(0xffffffffu, s0, (int)q);
-            if (j < rtotal) {
-                const uint32_t k = slot - lq;
-                s_id[w][j] = k < nq ? S.srd_btmp[bq + k] : P.nb + S.srd_stmp[sq + (k - nq)];
-            }
-        }
-        __syncwarp();
-        if (mine) {
-            uint32_t* ids = &s_id[w][loc - base];
-            for (uint32_t k = 1; k < n; ++k) {  // insertion sort of the cell's segment
-                const uint32_t x = ids[k];
-                uint32_t m = k;
-                while (m > 0 && ids[m - 1] > x) {
-                    ids[m] = ids[m - 1];
-                    --m;
-                }
-                ids[m] = x;
-            }
-        }
-        __syncwarp();
-        for (uint32_t j0 = 0; j0 < rtotal; j0 += 32u) {
-            const uint32_t j = j0 + lane, slot = base + (j < rtotal ? j : 0u);
-            const uint32_t q = (qpack >> (5u * (j0 >> 5))) & 31u;  // the cell of slot
-            const uint32_t gq = __shfl_sync(0xffffffffu, gdelta, (int)q);
-            if (j < rtotal) {
-                const uint32_t id = s_id[w][j];
-                S.srd_sorted_index[gq + slot] = id;
-                if (id < P.nb) {
-                    s_v[w][j] = bvel[id];
-                } else {
-                    s_v[w][j] = sv_old[id - P.nb];
-                    s_p[w][j] = sp_old[id - P.nb];
-                }
-            }
-        }
-        __syncwarp();
-        // per cell, by its lane: [lab isokinetic factor], mean velocity, rotation
-        // sign, [relative-velocity thermostat factor]
-        const bool lab = P.srd_thermo == NW_SRD_THERMO_REF_LAB;
-        const float ca = P.srd_cos_a;
-        float3 u = zero3();
-        float lam1 = 1.0f, sa = 0.0f, lam2 = 1.0f;
-        bool scale2 = false;
-        if (mine && n > 0) {
-            const uint32_t* ids = &s_id[w][loc - base];
-            const float4* V_ = &s_v[w][loc - base];
-            float E = 0.f;
-            if (lab)
-                for (uint32_t k = 0; k < n; ++k) {
-                    const float4 V = V_[k];
-                    const float3 v = f3(V);
-                    E += (0.5f * V.w) * dot3(v, v);
-                }
-            // reference isokinetic rule: lambda scales every member before the mean
-            lam1 = lab ? sqrtf(P.srd_kT / E) : 1.0f;
-            float M = 0.f;
-            for (uint32_t k = 0; k < n; ++k) {
-                const float4 V = V_[k];
-                u += V.w * (lab ? make_float3(lam1 * V.x, lam1 * V.y, lam1 * V.z) : f3(V));
-                M += V.w;
-            }
-            if (M > 0.f) {
-                const float inv = 1.0f / M;
-                u = u * inv;
-            }
-            // rotation by +alpha or -alpha with equal probability
-            const bool plus = u01(rng_draw(P, c, step, kRngSrdRot).x) > 0.5f;
-            sa = plus ? P.srd_sin_a : -P.srd_sin_a;
-            if (P.srd_thermo == NW_SRD_THERMO_CELL_REL) {
-                uint32_t nrot = 0;
-                float ke = 0.f;
-                for (uint32_t k = 0; k < n; ++k) {
-                    if (ids[k] < P.nb && !P.srd_rotate_beads) continue;
-                    const float4 V = V_[k];
-                    const float3 d = (lab ? make_float3(lam1 * V.x, lam1 * V.y, lam1 * V.z) : f3(V)) - u;
-                    const float rx = d.x * ca - d.y * sa;
-                    const float ry = d.x * sa + d.y * ca;
-                    ke += (0.5f * V.w) * (rx * rx + ry * ry);
-                    ++nrot;
-                }
-                if (nrot >= 2u && ke > 0.f) {
-                    lam2 = sqrtf(((float)(nrot - 1u) * P.srd_kT) / ke);
-                    scale2 = true;
-                }
-            }
-        }
-        // every member updated by the lane of its slot (the cell's factors from
-        // the cell's lane): rotation, thermostat, solvent streaming, and the
-        // member's destination in the new solvent storage (beads: none)
-        __syncwarp();
-        for (uint32_t j0 = 0; j0 < rtotal; j0 += 32u) {
-            const uint32_t j = j0 + lane, slot = base + (j < rtotal ? j : 0u);
-            const uint32_t q = (qpack >> (5u * (j0 >> 5))) & 31u;  // the cell of slot
-            const float3 uq = make_float3(__shfl_sync(0xffffffffu, u.x, (int)q), __shfl_sync(0xffffffffu, u.y, (int)q),
-                                          __shfl_sync(0xffffffffu, u.z, (int)q));
-            const float l1 = __shfl_sync(0xffffffffu, lam1, (int)q), saq = __shfl_sync(0xffffffffu, sa, (int)q);
-            const float l2 = __shfl_sync(0xffffffffu, lam2, (int)q);
-            const bool sc2 = __shfl_sync(0xffffffffu, (int)scale2, (int)q) != 0;
-            const uint32_t lq = __shfl_sync(0xffffffffu, loc, (int)q), nq = __shfl_sync(0xffffffffu, nbc, (int)q);
-            const uint32_t sq = __shfl_sync(0xffffffffu, s0, (int)q);
-            if (j < rtotal) {
-                const uint32_t id = s_id[w][j], k = slot - lq;
-                const bool is_bead = id < P.nb;
-                const float4 V = s_v[w][j];
-                float3 v = lab ? make_float3(l1 * V.x, l1 * V.y, l1 * V.z) : f3(V);
-                if (!is_bead || P.srd_rotate_beads) {
-                    const float3 d = v - uq;
-                    const float rx = d.x * ca - d.y * saq;
-                    const float ry = d.x * saq + d.y * ca;
-                    v = make_float3(uq.x + rx, uq.y + ry, uq.z + d.z);
-                    if (sc2) v = make_float3(uq.x + l2 * (v.x - uq.x), uq.y + l2 * (v.y - uq.y), v.z);
-                }
-                if (is_bead) {
-                    if (lab || P.srd_rotate_beads) bvel[id] = make_float4(v.x, v.y, v.z, V.w);
-                    s_id[w][j] = kEmpty;
-                } else {
-                    const float4 P4 = s_p[w][j];
-                    float3 p = f3(P4);
-                    const float3 dr = dt_srd * v;
-                    p += dr;
-                    apply_boundaries(P, p, v, dr, 0.0f);
-                    s_p[w][j] = make_float4(p.x, p.y, p.z, P4.w);
-                    s_v[w][j] = make_float4(v.x, v.y, v.z, V.w);
-                    s_id[w][j] = sq + (k - nq);
-                }
-            }
-        }
-        if (mine && valid && !big) S.srd_mean[c] = make_float4(u.x, u.y, u.z, 0.f);
-        __syncwarp();
-        for (uint32_t k = lane; k < rtotal; k += 32) {
-            const uint32_t d = s_id[w][k];
-            if (d != kEmpty) {
-                sp_new[d] = s_p[w][k];
-                sv_new[d] = s_v[w][k];
-            }
-        }
-        __syncwarp();
-        first = last + 1u;
-    }
-}
-
-__device__ __forceinline__ float warp_allsum(float x)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-}
-
-// The collision of srd_collide_kernel for one cell of more than kLaneCap
-// members, by one warp: members ranked by index in shared memory (the stable
-// order; beyond kBigCap members the bucket order, and the overflow is
-// reported), velocities gathered once into shared memory, sums as
-// lane-strided partials combined by a fixed butterfly (the same result on
-// every run), then the per-member update by all lanes.
-__global__ void __launch_bounds__(kBigWarps * 32) srd_collide_big_kernel(const DevParams P, const StepBuffers S,
-                                                                         uint32_t step_off, float dt_srd,
-                                                                         uint32_t buf_sel)
-{
-    __shared__ uint32_t s_in[kBigWarps][kBigCap];
-    __shared__ uint32_t s_id[kBigWarps][kBigCap];
-    __shared__ float4 s_v[kBigWarps][kBigCap];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t nbig = *S.srd_nbig;
-    const unsigned long long step = *S.step_base + step_off;
-    const uint32_t cur = buf_sel < 2u ? buf_sel : (uint32_t)(step & 1ull);
-    const uint32_t a = *S.scur;
-    const float4* __restrict__ sv_old = S.svel2[a];
-    const float4* __restrict__ sp_old = S.spos2[a];
-    float4* __restrict__ sv_new = S.svel2[a ^ 1u];
-    float4* __restrict__ sp_new = S.spos2[a ^ 1u];
-    float4* __restrict__ bvel = S.vel2[cur];
-    const bool lab = P.srd_thermo == NW_SRD_THERMO_REF_LAB;
-    const bool rel = P.srd_thermo == NW_SRD_THERMO_CELL_REL;
-    for (uint32_t q = blockIdx.x * kBigWarps + w; q < nbig; q += gridDim.x * kBigWarps) {
-        const uint32_t c = S.srd_big[q];
-        const uint32_t b0 = S.srd_boff[c], b1 = S.srd_boff[c + 1];
-        const uint32_t s0 = S.srd_soff[c], s1 = S.srd_soff[c + 1];
-        const uint32_t nbc = b1 - b0, n = nbc + (s1 - s0);
-        const uint32_t start = b0 + s0;
-        // beyond kBigCap members: bucket order, reported, bounded work
-        const bool fits = n <= kBigCap;
-        if (!fits && lane == 0) atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
-        auto raw = [&](uint32_t k) -> uint32_t {
-            return k < nbc ? S.srd_btmp[b0 + k] : P.nb + S.srd_stmp[s0 + (k - nbc)];
-        };
-        if (fits) {
-            for (uint32_t k = lane; k < n; k += 32) s_in[w][k] = raw(k);
-            __syncwarp();
-            for (uint32_t k = lane; k < n; k += 32) {
-                const uint32_t x = s_in[w][k];
-                uint32_t r = 0;
-                for (uint32_t j = 0; j < n; ++j) r += s_in[w][j] < x;
-                s_id[w][r] = x;
-            }
-            __syncwarp();
-        }
-        auto member = [&](uint32_t k) -> uint32_t { return fits ? s_id[w][k] : raw(k); };
-        auto vel_of = [&](uint32_t k, uint32_t id) -> float4 {
-            return fits ? s_v[w][k] : (id < P.nb ? bvel[id] : sv_old[id - P.nb]);
-        };
-        float E = 0.f;
-        for (uint32_t k = lane; k < n; k += 32) {
-            const uint32_t id = member(k);
-            S.srd_sorted_index[start + k] = id;
-            const float4 V = id < P.nb ? bvel[id] : sv_old[id - P.nb];
-            if (fits) s_v[w][k] = V;
-            E += (0.5f * V.w) * (V.x * V.x + V.y * V.y + V.z * V.z);
-        }
-        __syncwarp();
-        E = warp_allsum(E);
-        const float lam1 = lab ? sqrtf(P.srd_kT / E) : 1.0f;
-        float ux = 0.f, uy = 0.f, uz = 0.f, M = 0.f;
-        for (uint32_t k = lane; k < n; k += 32) {
-            const float4 V = vel_of(k, member(k));
-            const float sx = lab ? lam1 * V.x : V.x, sy = lab ? lam1 * V.y : V.y, sz = lab ? lam1 * V.z : V.z;
-            ux += V.w * sx;
-            uy += V.w * sy;
-            uz += V.w * sz;
-            M += V.w;
-        }
-        ux = warp_allsum(ux);
-        uy = warp_allsum(uy);
-        uz = warp_allsum(uz);
-        M = warp_allsum(M);
-        if (M > 0.f) {
-            const float inv = 1.0f / M;
-            ux *= inv;
-            uy *= inv;
-            uz *= inv;
-        }
-        const bool plus = u01(rng_draw(P, c, step, kRngSrdRot).x) > 0.5f;
-        const float sa = plus ? P.srd_sin_a : -P.srd_sin_a, ca = P.srd_cos_a;
-        float lam2 = 1.0f;
-        bool scale2 = false;
-        if (rel) {
-            float ke = 0.f, nrot = 0.f;
-            for (uint32_t k = lane; k < n; k += 32) {
-                if (member(k) < P.nb && !P.srd_rotate_beads) continue;
-                const float4 V = vel_of(k, member(k));
-                const float dx = (lab ? lam1 * V.x : V.x) - ux, dy = (lab ? lam1 * V.y : V.y) - uy;
-                const float rx = dx * ca - dy * sa, ry = dx * sa + dy * ca;
-                ke += (0.5f * V.w) * (rx * rx + ry * ry);
-                nrot += 1.f;
-            }
-            ke = warp_allsum(ke);
-            nrot = warp_allsum(nrot);
-            if (nrot >= 2.f && ke > 0.f) {
-                lam2 = sqrtf(((nrot - 1.f) * P.srd_kT) / ke);
-                scale2 = true;
-            }
-        }
-        for (uint32_t k = lane; k < n; k += 32) {
-            const uint32_t id = member(k);
-            const bool is_bead = id < P.nb;
-            const float4 V = vel_of(k, id);
-            float3 v = lab ? make_float3(lam1 * V.x, lam1 * V.y, lam1 * V.z) : f3(V);
-            if (!is_bead || P.srd_rotate_beads) {
-                const float dx = v.x - ux, dy = v.y - uy, dz = v.z - uz;
-                const float rx = dx * ca - dy * sa, ry = dx * sa + dy * ca;
-                v = make_float3(ux + rx, uy + ry, uz + dz);
-                if (scale2) v = make_float3(ux + lam2 * (v.x - ux), uy + lam2 * (v.y - uy), v.z);
-            }
-            if (is_bead) {
-                if (lab || P.srd_rotate_beads) bvel[id] = make_float4(v.x, v.y, v.z, V.w);
-            } else {
-                const float4 P4 = sp_old[id - P.nb];
-                float3 p = f3(P4);
-                const float3 dr = dt_srd * v;
-                p += dr;
-                apply_boundaries(P, p, v, dr, 0.0f);
-                const uint32_t dst = s0 + (k - nbc);
-                sp_new[dst] = make_float4(p.x, p.y, p.z, P4.w);
-                sv_new[dst] = make_float4(v.x, v.y, v.z, V.w);
-            }
-        }
-        if (lane == 0) S.srd_mean[c] = make_float4(ux, uy, uz, 0.f);
-        __syncwarp();
-    }
-}
-
-// The collision just written the solvent to the other buffer.
-__global__ void srd_flip_kernel(uint32_t* scur) { *scur ^= 1u; }
 
 __global__ void advance_step_kernel(unsigned long long* step_base, unsigned long long k) { *step_base += k; }
 

@@ -11,16 +11,57 @@
 //   pair_*          pair forces over the 3x3(x3) neighbour cells
 // The cell-list and Verlet strategies (nw_fused_impl.cuh) run one fused kernel
 // per step instead.  Every srd_gap steps an SRD collision adds seven:
-//   srd_hash, chunk_sum and scan_cells (bead and solvent buckets side by
-//   side), srd_scatter, srd_collide, srd_collide_big, srd_flip.
+//   srd_bead_hash, srd_hash, chunk_sum and scan_cells (bead and solvent counts
+//   side by side), srd_scatter, srd_collide, srd_collide_big (nw_srd.cu).
 //
 // No float atomics are used anywhere: every output element has exactly one
 // writer, so repeated runs are bit-identical.
 #pragma once
 
+#include <utility>
+
 #include "nw_device.cuh"
 
 namespace nw {
+
+// Programmatic dependent launch: the step kernels are launched with the
+// stream-serialisation attribute relaxed, so that a kernel's blocks may be
+// scheduled while the previous kernel's last blocks still run.  Each step
+// kernel first waits (griddepcontrol.wait) until the previous kernel has
+// completed and its writes are visible, exactly the stream order, and then
+// lets the next launch begin.  Launched without the attribute both
+// instructions return at once.  NW_PDL=0 builds plain launches.
+#ifndef NW_PDL
+#define NW_PDL 1
+#endif
+__device__ __forceinline__ void pdl_enter()
+{
+#if NW_PDL
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
+template <class... KArgs, class... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, uint32_t block, size_t smem, cudaStream_t s,
+                       Args&&... args)
+{
+#if NW_PDL
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+#else
+    kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
+#endif
+}
 
 // Beyond these occupancies a cell is reported (NW_EFLAG_CELL_OVERFLOW) and
 // processed with bounded work; physical states never get close.
@@ -53,11 +94,14 @@ struct StepBuffers {
     uint32_t *nbr, *nnb, *vstate;
     uint32_t *cell_count, *cell_offset, *cell_start, *cell_end, *chunk_count;
     float4 *sorted_pos, *sorted_vel, *sorted_tan;
-    // SRD collision: per-particle cell hash and slot (beads [0, nb), solvent
-    // [nb, ntotal)); beads and solvent are bucketed separately (a cell's
-    // members in the stable order are its beads, then its solvent)
+    // SRD collision: per-particle cell hash (beads [0, nb), solvent
+    // [nb, ntotal)) and, where the solvent is bucketed, slot; a cell's members
+    // in the stable order are its beads, then its solvent
     uint32_t *srd_hash, *srd_slot, *srd_btmp, *srd_stmp, *srd_sorted_index;
-    uint32_t *srd_bcount, *srd_scount, *srd_boff, *srd_soff, *srd_bchunk, *srd_schunk;
+    uint32_t *srd_bcount, *srd_scount, *srd_boff, *srd_bchunk, *srd_schunk;
+    uint32_t* srd_soff2[2];               // solvent cell offsets of buffer spos2[k]
+    uint32_t *srd_btab, *srd_bhead, *srd_bnext;  // the beads of each cell: a few in a table, more in a linked list
+    uint32_t* srd_state;                  // kSrdWords words (see kSrdGeo)
     uint32_t *srd_start, *srd_end;
     float4* srd_mean;
     // SRD cells of more than kLaneCap members, handed to
@@ -234,19 +278,22 @@ __global__ void __launch_bounds__(1024) filament_pass_kernel(const DevParams P, 
 // offset[c] = exclusive prefix, offset[ncells] = total; start/end in the
 // reference's format (0xffffffff for empty cells); counts are reset to zero.
 // A grid two blocks high scans a second array (count2, chunk_count2 ->
-// offset2; no bounds) in its second row.
+// offset2, or offset2_alt where *alt is set; no bounds) in its second row.
 template <bool kBounds>
 __global__ void __launch_bounds__(512) scan_cells_kernel(uint32_t* __restrict__ count,
                                                          const uint32_t* __restrict__ chunk_count, uint32_t ncells,
                                                          uint32_t* __restrict__ offset, uint32_t* __restrict__ start,
                                                          uint32_t* __restrict__ end, uint32_t* __restrict__ count2,
                                                          const uint32_t* __restrict__ chunk_count2,
-                                                         uint32_t* __restrict__ offset2)
+                                                         uint32_t* __restrict__ offset2,
+                                                         uint32_t* __restrict__ offset2_alt,
+                                                         const uint32_t* __restrict__ alt)
 {
+    pdl_enter();
     if (blockIdx.y) {
         count = count2;
         chunk_count = chunk_count2;
-        offset = offset2;
+        offset = alt && *alt ? offset2_alt : offset2;
     }
     const bool bounds = kBounds && blockIdx.y == 0;
     __shared__ uint32_t s_w[16];
@@ -555,23 +602,28 @@ __device__ __forceinline__ float3 srd_shift_of(const DevParams& P, unsigned long
                        P.dim >= 3 ? (P.srd_shift_lo + u01(x.z)) * P.srd_cell[2] : 0.0f);
 }
 
-// calcHashD(srd = true) over beads and solvent + counting-sort slot.
-__global__ void __launch_bounds__(256) srd_hash_kernel(const DevParams P, const StepBuffers S, uint32_t step_off,
-                                                       int shift_from_step, float3 shift, uint32_t buf_sel);
+// ---- SRD collision (nw_srd.cu) -----------------------------------------------------
+//
+// Words of StepBuffers::srd_state.  The solvent of buffer k lies in the cell
+// order of the collision that wrote it: kSrdGeo + 8 k holds that collision's
+// grid shift (three floats), the largest displacement of its streaming in
+// cells of any axis (float bits) and a word that is 1 while nothing else has
+// written the buffer's positions since.  The rest describes the collision in
+// progress: the buffer it reads, whether the cell order of that buffer bounds
+// where each cell's members can be (`ordered`), and per axis the lowest cell
+// step of a particle between the two collisions' grids and their number.
+enum : uint32_t {
+    kSrdGeo = 0,       // [2][8]: shift x, y, z, largest step, ordered
+    kSrdStep = 3,      // within a geo entry
+    kSrdHeld = 4,      // within a geo entry
+    kSrdSrc = 16,      // solvent buffer read by the collision in progress
+    kSrdOrdered = 17,  // 1: members are found through the old cell order
+    kSrdLo = 18,       // [3] lowest cell step per axis
+    kSrdN = 21,        // [3] number of cell steps per axis
+    kSrdWords = 24
+};
+constexpr int kSrdSteps = 4;  // cell steps per axis the ordered path takes
 
-// SRD collision, a warp per 32 consecutive cells staged in shared memory,
-// one cell per thread: members in stable (index) order, then the reference's
-// isokinetic thermostat (particles_kernel_impl.cuh:605-637) or none, the
-// mass-weighted cell mean (:560-594), the +/- alpha rotation of (v - u)
-// (:640-691), the relative-velocity thermostat when selected, and the
-// solvent's ballistic streaming by dt_srd (solvent_integrator, :145-205).
-__global__ void __launch_bounds__(128, 8) srd_collide_kernel(const DevParams P, const StepBuffers S, uint32_t step_off,
-                                                             float dt_srd, uint32_t buf_sel);
-
-__global__ void __launch_bounds__(256) srd_scatter_kernel(const DevParams P, const StepBuffers S);
-// One warp per SRD cell of the srd_big list (grid-stride over the list).
-__global__ void __launch_bounds__(128) srd_collide_big_kernel(const DevParams P, const StepBuffers S,
-                                                              uint32_t step_off, float dt_srd, uint32_t buf_sel);
 // Tuning of the collision's two paths (overridable at compile time):
 // blocks of srd_collide_big_kernel, and the largest cell one lane of
 // srd_collide_kernel collides (larger cells go to the warp-per-cell kernel).
@@ -585,7 +637,6 @@ constexpr uint32_t kSrdBigBlocks = NW_SRD_BIG_BLOCKS;
 constexpr uint32_t kLaneCap = NW_SRD_LANE_CAP;  // members of a cell collided by one lane of srd_collide_kernel
 constexpr uint32_t kBigWarps = 4;        // warps (cells at a time) per block of srd_collide_big_kernel
 constexpr uint32_t kBigCap = 384;        // members of a cell ordered exactly by srd_collide_big_kernel
-__global__ void srd_flip_kernel(uint32_t* scur);
 
 __global__ void advance_step_kernel(unsigned long long* step_base, unsigned long long k);
 

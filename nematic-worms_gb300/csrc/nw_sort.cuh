@@ -70,7 +70,7 @@ inline void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, const R
         radix_hist_kernel<<<nblocks, 256, 0, s>>>(ki, n, shift, S.ghist, nblocks);
         chunk_sum_kernel<<<nchunks, 512, 0, s>>>(S.ghist, m, S.chunk, nullptr, nullptr);
         scan_cells_kernel<false><<<nchunks, 512, 0, s>>>(S.ghist, S.chunk, m, S.goffset, nullptr, nullptr, nullptr,
-                                                          nullptr, nullptr);
+                                                          nullptr, nullptr, nullptr, nullptr);
         radix_scatter_kernel<<<nblocks, 256, 0, s>>>(ki, vi, ko, vo, n, shift, S.goffset, nblocks);
         uint32_t* t = ki;
         ki = ko;
