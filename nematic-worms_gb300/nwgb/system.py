@@ -218,14 +218,15 @@ class System:
         defects first, each sign in order of its first grid cell.  cell_size
         is the reference's ``--cellsize`` (default 2); min_image takes bead
         tangents through the periodic boundary (the reference does not)."""
-        buf = (abi.NwDefect * max_defects)()
+        buf = np.empty(max_defects, dtype=abi.DEFECT_DTYPE)
         n = C.c_int()
         flags = abi.NW_DEFECT_MIN_IMAGE if min_image else 0
-        check(self.lib.nw_find_defects(self._h, float(cell_size), flags, buf, max_defects, C.byref(n)),
+        check(self.lib.nw_find_defects(self._h, float(cell_size), flags, buf.ctypes.data, max_defects,
+                                       C.byref(n)),
               "nw_find_defects")
         if n.value > max_defects:
             return self.find_defects(cell_size, min_image, n.value)
-        return np.frombuffer(buf, dtype=abi.DEFECT_DTYPE, count=n.value).copy()
+        return buf[:n.value].copy()
 
     def sample_defects(self, beads, radius: float = 10.0, min_image: bool = False) -> np.ndarray:
         """Winding value around the position of each bead in `beads`
