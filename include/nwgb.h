@@ -169,9 +169,7 @@ typedef struct NwConfig {
  *              pair pass otherwise.  Same forces as CELL_LISTS up to the
  *              order of the FP32 sums.
  *  AUTO        VERLET for WCA_WORMS, SORTED for REF_DEM (whose pair set is
- *              all beads of the neighbour cells, not a radius; its sorted
- *              pair pass on a single z layer runs cell-tiled in shared
- *              memory). */
+ *              all beads of the neighbour cells, not a radius). */
 typedef enum {
     NW_STRATEGY_AUTO = 0,
     NW_STRATEGY_SORTED = 1,

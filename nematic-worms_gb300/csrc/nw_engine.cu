@@ -152,30 +152,28 @@ uint64_t enqueue_bead_step(const DevParams& P, const StepBuffers& B, uint32_t nc
     const uint32_t beads = fpb * P.L;
     const uint32_t threads = (beads + 31u) & ~31u;
     const size_t smem = (size_t)beads * sizeof(float4) * (P.reverse_on ? 3u : 1u);
+    const uint32_t blocks = cdiv(P.nb, 256);
+    uint32_t* const none = nullptr;
     NW_MARK("filament_pass");
-    filament_pass_kernel<<<cdiv(P.nf, fpb), threads, smem, s>>>(P, B, step_off, dt, fpb);
+    launch_pdl(filament_pass_kernel, cdiv(P.nf, fpb), threads, smem, s, P, B, step_off, dt, fpb);
     NW_MARK("chunk_sum");
-    chunk_sum_kernel<<<nchunks, 512, 0, s>>>(B.cell_count, P.ncells, B.chunk_count, nullptr, nullptr);
+    launch_pdl(chunk_sum_kernel, nchunks, 512, 0, s, B.cell_count, P.ncells, B.chunk_count, none, none);
     NW_MARK("scan_cells");
-    scan_cells_kernel<true><<<nchunks, 512, 0, s>>>(B.cell_count, B.chunk_count, P.ncells, B.cell_offset, B.cell_start,
-                                                    B.cell_end, nullptr, nullptr, nullptr, nullptr, nullptr);
+    launch_pdl(scan_cells_kernel<true>, nchunks, 512, 0, s, B.cell_count, B.chunk_count, P.ncells, B.cell_offset,
+               B.cell_start, B.cell_end, none, none, none, none, none);
     NW_MARK("scatter");
-    scatter_kernel<<<cdiv(P.nb, 256), 256, 0, s>>>(B.hash, B.slot, B.cell_offset, B.tmp_index, P.nb);
+    launch_pdl(scatter_kernel, blocks, 256, 0, s, B.hash, B.slot, B.cell_offset, B.tmp_index, P.nb);
     if (P.model == NW_MODEL_REF_DEM) {
         NW_MARK("stable_gather");
-        stable_gather_kernel<true><<<cdiv(P.nb, 256), 256, 0, s>>>(P, B);
+        launch_pdl(stable_gather_kernel<true>, blocks, 256, 0, s, P, B);
         NW_MARK("pair_ref");
-        if (P.grid[2] == 1u) {
-            const uint32_t tiles = cdiv(P.grid[0], kRefTX) * cdiv(P.grid[1], kRefTY);
-            pair_ref_tiled_kernel<<<tiles, kRefThreads, kRefSmem, s>>>(P, B);
-        } else {
-            pair_ref_kernel<<<cdiv(P.nb, 256), 256, 0, s>>>(P, B);
-        }
+        if (P.grid[2] == 1u) launch_pdl(pair_ref_runs_kernel, cdiv((uint64_t)P.nb * kRefG, 256), 256, 0, s, P, B);
+        else launch_pdl(pair_ref_kernel, blocks, 256, 0, s, P, B);
     } else {
         NW_MARK("stable_gather");
-        stable_gather_kernel<false><<<cdiv(P.nb, 256), 256, 0, s>>>(P, B);
+        launch_pdl(stable_gather_kernel<false>, blocks, 256, 0, s, P, B);
         NW_MARK("pair_wca");
-        pair_wca_kernel<<<cdiv(P.nb, 256), 256, 0, s>>>(P, B);
+        launch_pdl(pair_wca_kernel, blocks, 256, 0, s, P, B);
     }
     return 6;
 }
@@ -407,7 +405,7 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
     }
     if (!state_marked) mark_state();
     if (prof) prof->mark("advance_step");
-    advance_step_kernel<<<1, 1, 0, s->stream>>>(s->B.step_base, (unsigned long long)nsteps);
+    launch_pdl(advance_step_kernel, 1, 1, 0, s->stream, s->B.step_base, (unsigned long long)nsteps);
     if (prof) prof->end();
     return launches + 1;
 }
@@ -614,14 +612,6 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         return NW_ERR_CUDA;
     }
     s->stream = s->own_stream;
-    // the cell-tiled REF_DEM pair pass stages more than the default 48 KB
-    if (cudaFuncSetAttribute(pair_ref_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRefSmem) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        cudaStreamDestroy(s->own_stream);
-        delete s;
-        return NW_ERR_CUDA;
-    }
     s->lists = effective_strategy(*cfg) != NW_STRATEGY_SORTED;
     const DevParams P0 = make_dev_params(*cfg, cfg->dt);
     s->vl = P0.vl_on != 0;

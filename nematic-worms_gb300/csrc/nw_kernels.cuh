@@ -411,18 +411,26 @@ __device__ __forceinline__ uint32_t bucket_rank(const uint32_t* __restrict__ tmp
 template <bool kRef>
 __global__ void __launch_bounds__(256) stable_gather_kernel(const DevParams P, const StepBuffers S)
 {
+    pdl_enter();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= P.nb) return;
     const uint32_t i = S.tmp_index[q];
     const uint32_t h = S.hash[i];
+    // the bead's data on its way while its rank is found
+    const float4 pos = S.pos[i];
+    float4 vel = pos, tan = pos;
+    if (kRef) {
+        vel = S.vel[i];
+        tan = S.tangent[i];
+    }
     const uint32_t lo = S.cell_offset[h], hi = S.cell_offset[h + 1];
     const uint32_t d = lo + bucket_rank(S.tmp_index, lo, hi, i, q, S.err);
     S.sorted_index[d] = i;
     S.sorted_hash[d] = h;
-    S.sorted_pos[d] = S.pos[i];
+    S.sorted_pos[d] = pos;
     if (kRef) {
-        S.sorted_vel[d] = S.vel[i];
-        S.sorted_tan[d] = S.tangent[i];
+        S.sorted_vel[d] = vel;
+        S.sorted_tan[d] = tan;
     }
 }
 
@@ -499,17 +507,10 @@ __device__ __forceinline__ float3 ref_cell_sum(const DevParams& P, const StepBuf
 // z, y, x order, which reproduces the reference's accumulation exactly.
 __global__ void __launch_bounds__(256) pair_ref_kernel(const DevParams P, const StepBuffers S);
 
-// REF_DEM pair pass over tiles of kRefTX x kRefTY cells of a single z layer
-// (layout in nw_kernels.cu).  Grid: ceil(gx / kRefTX) * ceil(gy / kRefTY)
-// blocks of kRefThreads with kRefSmem bytes of dynamic shared memory (above
-// the default 48 KB: the kernel's attribute is raised when a system is made).
-constexpr uint32_t kRefTX = 32, kRefTY = 4, kRefG = 4, kRefThreads = 256;
-constexpr uint32_t kRefHX = kRefTX + 2, kRefHalo = kRefHX * (kRefTY + 2);
-constexpr uint32_t kRefStage = 1024;
-constexpr size_t kRefSmem = (size_t)kRefStage * (3 * 16 + 2 * 4) + (size_t)(2 * kRefHalo + 1) * 4;
-static_assert(kRefHalo <= kRefThreads, "one thread per halo cell");
+// REF_DEM pair pass of a single z layer, kRefG lanes a bead (nw_kernels.cu).
+constexpr uint32_t kRefG = 2;
 static_assert(32 % kRefG == 0, "lane groups within a warp");
-__global__ void __launch_bounds__(kRefThreads) pair_ref_tiled_kernel(const DevParams P, const StepBuffers S);
+__global__ void __launch_bounds__(256) pair_ref_runs_kernel(const DevParams P, const StepBuffers S);
 
 // Neighbour cell c + o (o in -1..1) of an axis of G cells as the
 // distinct-cell visit takes it: wrapped on periodic axes, absent beyond a

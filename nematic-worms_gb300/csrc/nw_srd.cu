@@ -907,13 +907,12 @@ uint64_t enqueue_srd(const DevParams& P, const StepBuffers& B, uint32_t srd_nchu
                     : periodic && P.srd_thermo == NW_SRD_THERMO_REF_LAB && !P.srd_rotate_beads
                         ? srd_collide_kernel<kLab>
                         : srd_collide_kernel<kAny>;
+    const bool dense = (uint64_t)P.ntotal > 8ull * P.srd_ncells;
     launch_pdl(collide, cdiv(P.srd_ncells, kCollideWarps * 32), kCollideWarps * 32, 0, s, P, B, step_off, dt_srd,
                buf_sel);
     NW_MARK("srd_collide_big");
     // few cells of a dilute solvent are big: a block for 1,024 cells there
-    const uint32_t big_blocks = (uint64_t)P.ntotal > 8ull * P.srd_ncells
-                                    ? cdiv(P.srd_ncells, kBigWarps)
-                                    : std::max(8u, cdiv(P.srd_ncells, 1024));
+    const uint32_t big_blocks = dense ? cdiv(P.srd_ncells, kBigWarps) : std::max(8u, cdiv(P.srd_ncells, 1024));
     launch_pdl(srd_collide_big_kernel, std::min(kSrdBigBlocks, big_blocks), kBigWarps * 32, 0, s, P, B, step_off,
                dt_srd, buf_sel);
     return 7;
