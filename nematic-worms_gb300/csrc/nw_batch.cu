@@ -52,6 +52,7 @@ struct nw_batch {
     bool use_graphs = true, vl = false, vl_dirty = true, lists_dirty = true;
     bool tan_stale = false;  // tangents of lazy replicas (pro_flags) computed when read
     bool planar = false;     // every replica is two-dimensional (the planar kernels)
+    bool packed = false;     // every replica keeps its state packed between the updates of a call
     std::vector<BatchGraph> graphs;
 };
 
@@ -174,6 +175,7 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
     std::vector<uint32_t> block_rep;
     uint64_t cells = 0, nbr_words = 0;
     b->vl = false;
+    b->packed = true;
     for (int r = 0; r < b->R; ++r) {
         NwConfig c = b->cfg[r];
         c.strategy = t.strategy;
@@ -193,6 +195,7 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
         e.nblk = c.num_filaments ? cdivu(c.num_filaments, fpb) : 0u;
         for (uint32_t k = 0; k < e.nblk; ++k) block_rep.push_back((uint32_t)r);
         cells += e.P.lncells;
+        b->packed = b->packed && packs(e.P);
         if (e.P.vl_on) {
             b->vl = true;
             nbr_words += (uint64_t)e.P.vl_cap * b->nb[r];
@@ -260,19 +263,22 @@ uint64_t enqueue(nw_batch* b, int nsteps)
 {
     if (b->blocks == 0) return 0;
     uint64_t launches = 0;
-    auto L = [&](int mode, uint32_t off) {
+    auto L = [&](int mode, uint32_t off, uint32_t packed) {
         launch_batch(mode, b->d_slots, b->d_block_rep, b->blocks, b->threads, b->smem, b->cap, b->B, off, b->planar,
-                     b->stream);
+                     packed, b->stream);
         ++launches;
     };
-    L(kBatchPro, 0u);
-    if (b->vl) L(kBatchList, 0u);
+    // every update but the last leaves its state packed
+    auto in = [&](int j) { return b->packed && j < nsteps - 1 ? kPackedIn : 0u; };
+    auto out = [&](int j) { return b->packed && j < nsteps - 1 ? kPackedOut : 0u; };
+    L(kBatchPro, 0u, out(0));
+    if (b->vl) L(kBatchList, 0u, in(0));
     for (int j = 0; j < nsteps; ++j) {
         if (j == nsteps - 1) {
-            L(kBatchEpi, (uint32_t)j);
+            L(kBatchEpi, (uint32_t)j, 0u);
         } else {
-            L(kBatchFused, (uint32_t)j);
-            if (b->vl) L(kBatchList, (uint32_t)(j + 1));
+            L(kBatchFused, (uint32_t)j, in(j) | out(j + 1));
+            if (b->vl) L(kBatchList, (uint32_t)(j + 1), in(j + 1));
         }
     }
     advance_step_kernel<<<1, 1, 0, b->stream>>>(b->B.step_base, (unsigned long long)nsteps);
@@ -383,6 +389,10 @@ nw_status nw_batch_create(const NwConfig* replicas, int n, nw_batch** out)
     }
     A(balloc(b->state_allocs, &B.force, nbt));
     A(balloc(b->state_allocs, &B.force_old, nbt));
+    if (b->planar) {
+        for (int k = 0; k < 2; ++k) A(balloc(b->state_allocs, &B.pk[k], nbt));
+        A(balloc(b->state_allocs, &B.pf, nbt));
+    }
     A(balloc(b->state_allocs, &B.err, 4));
     A(balloc(b->state_allocs, &B.step_base, 1));
     cudaError_t e = cudaSuccess;

@@ -57,6 +57,10 @@ struct DevParams {
     float vl_half_skin;  // lists stay valid while the displacement bound is below this
     uint32_t vl_cap;     // neighbours per bead list
     float ibox[3];       // 1 / box on periodic axes, 0 on the others (min_image_near)
+    // beads between these coordinates have no listed neighbour across a
+    // periodic boundary (unbounded on the other axes)
+    float vl_lo[3], vl_hi[3];
+    uint32_t L_m, L_k;   // multiply-shift divisor by L
     // SRD grid: multiply-shift divisors by its x extent and its layer, cells
     // per unit length (0 on axes of one cell), the box's middle and the
     // distance from it up to which positions count as near the box, and whether
@@ -428,6 +432,13 @@ __device__ __forceinline__ void apply_boundaries(const DevParams& P, float3& p, 
             }
         }
     }
+}
+
+// n mod 3: 2^32 is 1 mod 3, so the halves' remainders add.
+__device__ __forceinline__ uint32_t mod3(unsigned long long n)
+{
+    const uint32_t r = (uint32_t)(n >> 32) % 3u + (uint32_t)n % 3u;
+    return r >= 3u ? r - 3u : r;
 }
 
 // Filament of a bead index (beads are stored filament by filament).

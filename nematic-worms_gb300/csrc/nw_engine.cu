@@ -80,6 +80,13 @@ DevParams make_dev_params(const NwConfig& c, float dt)
     P.vl_r2 = rl * rl;
     P.vl_half_skin = 0.5f * skin;
     P.vl_cap = c.neighbor_capacity ? c.neighbor_capacity : 32u;
+    fast_div_params(P.L ? P.L : 1u, P.L_m, P.L_k);
+    for (int a = 0; a < 3; ++a) {
+        // a listed pair stays within lj_rcut + 2 skin (and a little for rounding)
+        const float reach = (c.lj_rcut + 2.0f * skin) * 1.001f + 1e-5f * c.box[a];
+        P.vl_lo[a] = P.bnd[a] == NW_PERIODIC ? P.origin[a] + reach : -INFINITY;
+        P.vl_hi[a] = P.bnd[a] == NW_PERIODIC ? P.origin[a] + P.box[a] - reach : INFINITY;
+    }
     P.lncells = 1;
     for (int a = 0; a < 3; ++a) {
         if (P.vl_on) {
@@ -370,20 +377,26 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
         // and its pair pass, keeping the pair/integrate chain fused; REF_DEM
         // pair forces read velocities, so its collision follows the pair pass.
         const bool wca = P.model == NW_MODEL_WCA_WORMS;
-        auto list = [&](uint32_t j) {
+        auto hit = [&](int j) { return srd && ((first_step + (uint64_t)j) % gap) == 0; };
+        // updates that leave their state packed: neither read by a collision nor the last
+        const bool pack = packs(P) && s->B.pf;  // no packed buffers where reversal was switched off later
+        auto packed = [&](int j) { return pack && j < nsteps - 1 && !hit(j); };
+        uint32_t from = 1u;  // parity of the last update in the API's arrays (-1: the state before the call)
+        auto list = [&](int j) {
+            if (!packed(j)) from = (uint32_t)j & 1u;
             if (!P.vl_on) return;
             NW_MARK("bead_list");
-            launches += launch_bead_list(P, s->B, j, s->stream);
+            launches += launch_bead_list(P, s->B, (uint32_t)j, packed(j), s->stream);
         };
         auto collide = [&](uint32_t j) {
             launches += enqueue_srd(P, s->B, s->srd_nchunks, j, dt_srd, 1, make_float3(0.f, 0.f, 0.f), s->stream,
                                     prof, 2u);
         };
         NW_MARK("bead_pro");
-        launches += launch_bead_pro(P, s->B, 0u, dt, s->stream);
-        list(0u);
+        launches += launch_bead_pro(P, s->B, 0u, dt, packed(0) ? kPackedOut : 0u, s->stream);
+        list(0);
         for (int j = 0; j < nsteps; ++j) {
-            const bool srd_now = srd && ((first_step + (uint64_t)j) % gap) == 0;
+            const bool srd_now = hit(j);
             if (srd_now && wca) collide((uint32_t)j);
             if (j == nsteps - 1 || (srd_now && !wca)) {
                 // WCA: the last update's pair pass changes forces only
@@ -393,13 +406,15 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
                 if (srd_now && !wca) collide((uint32_t)j);
                 if (j < nsteps - 1) {
                     NW_MARK("bead_pro");
-                    launches += launch_bead_pro(P, s->B, (uint32_t)(j + 1), dt, s->stream);
-                    list((uint32_t)(j + 1));
+                    launches += launch_bead_pro(P, s->B, (uint32_t)(j + 1), dt, 0u, s->stream);
+                    list(j + 1);
                 }
             } else {
                 NW_MARK("bead_fused");
-                launches += launch_bead_fused(P, s->B, (uint32_t)j, dt, s->stream);
-                list((uint32_t)(j + 1));
+                launches += launch_bead_fused(P, s->B, (uint32_t)j, dt,
+                                              (packed(j) ? kPackedIn : 0u) | (packed(j + 1) ? kPackedOut : 0u), from,
+                                              s->stream);
+                list(j + 1);
             }
         }
     }
@@ -689,6 +704,10 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         const size_t LC = P0.lncells > C ? P0.lncells : C;
         for (int k = 0; k < 3; ++k) A(alloc_n(s, &B.lcount[k], LC + 8));
         for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.lslot[k], LC * B.cap + 8));
+    }
+    if (packs(P0)) {
+        for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.pk[k], nb));
+        A(alloc_n(s, &B.pf, nb));
     }
     if (s->vl) {
         A(alloc_n(s, &B.nbr, (size_t)P0.vl_cap * nb + 8));

@@ -15,6 +15,21 @@ __host__ __device__ __forceinline__ uint32_t pro_flags(const DevParams& P)
 {
     return P.model == NW_MODEL_WCA_WORMS && P.L > 3u ? kProLazyTangent : 0u;
 }
+// Within one call, the bead state of planar Verlet systems between updates is
+// packed: two float4 a bead (x, y, velocity; partial and previous force)
+// instead of four, since z, the radius and the mass stay as they are and the
+// forces have z = 0.  The first update reads and the last writes the API's
+// arrays, and so does an update with a collision, which reads and changes bead
+// velocities in them.  A kernel that leaves the packed form takes z, radius
+// and mass from the buffer of the last update that wrote the API's arrays.
+// 40 updates of 2,000,000 beads: 3.76 -> 3.15 ms (128 of 306 MB a launch less),
+// ten of 400,000 with SRD 327 -> 301 us, 20 of 64 replicas 1.23 -> 1.12 ms.
+constexpr uint32_t kPackedIn = 1u, kPackedOut = 2u;
+__host__ __device__ __forceinline__ bool packs(const DevParams& P)
+{
+    return planar_system(P) && P.vl_on && !P.reverse_on && P.lgrid[2] == 1u && P.L <= 256u &&
+           (pro_flags(P) & kProLazyTangent) != 0u;
+}
 // Tangents of the current positions as the pro part computes them.
 uint64_t launch_bead_tangents(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s);
 
@@ -22,14 +37,20 @@ uint64_t launch_bead_tangents(const DevParams& P, const float4* pos, float4* tan
 uint32_t list_filaments_per_block(uint32_t L, uint32_t nf);
 
 // pro(n) with n = *step_base + off: integrate .. hash, insert into list n.
-uint64_t launch_bead_pro(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s);
+// packed: kPackedOut or 0.
+uint64_t launch_bead_pro(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                         cudaStream_t s);
 // Verlet systems: the cell list of update n, built only when the pair pass
 // of update n rebuilds the neighbour lists (launch after the pro part of n).
-uint64_t launch_bead_list(const DevParams& P, const StepBuffers& B, uint32_t off, cudaStream_t s);
+// packed: whether update n left its state packed.
+uint64_t launch_bead_list(const DevParams& P, const StepBuffers& B, uint32_t off, bool packed, cudaStream_t s);
 // epi(n): pair forces from list n; force = complete F_n.
 uint64_t launch_bead_epi(const DevParams& P, const StepBuffers& B, uint32_t off, cudaStream_t s);
-// epi(n) followed by pro(n+1) in one kernel.
-uint64_t launch_bead_fused(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s);
+// epi(n) followed by pro(n+1) in one kernel; packed: kPackedIn | kPackedOut;
+// from: parity of the offset of the last update in the API's arrays (-1, the
+// state before the call, is odd).
+uint64_t launch_bead_fused(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                           uint32_t from, cudaStream_t s);
 
 // ---- batched replicas (nw_batch.cu) ------------------------------------------
 
@@ -56,15 +77,18 @@ enum BatchMode { kBatchPro = 0, kBatchEpi = 1, kBatchFused = 2, kBatchList = 3 }
 // the batch's base pointers; `threads` >= every replica's fpb * L; planar =
 // every replica is a planar system.
 void launch_batch(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks, uint32_t threads,
-                  size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off, bool planar, cudaStream_t s);
+                  size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off, bool planar, uint32_t packed,
+                  cudaStream_t s);
 
 // The two-component launches (nw_fused_planar.cu) behind the launchers above.
-uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s);
+uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                                cudaStream_t s);
 uint64_t launch_bead_tangents_planar(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s);
 uint64_t launch_bead_epi_planar(const DevParams& P, const StepBuffers& B, uint32_t off, cudaStream_t s);
-uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s);
+uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                                  uint32_t from, cudaStream_t s);
 void launch_batch_planar(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks,
                          uint32_t threads, size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off,
-                         cudaStream_t s);
+                         uint32_t packed, cudaStream_t s);
 
 }  // namespace nw

@@ -19,6 +19,8 @@
 // order as with the sorted arrays, and runs are bit-identical.
 #pragma once
 
+#include <type_traits>
+
 #include "nw_fused.cuh"
 
 namespace nw {
@@ -212,7 +214,19 @@ __device__ __forceinline__ float3 ref_list_force(const DevParams& P, const float
 __device__ __forceinline__ float vl_bound(const StepBuffers& S, unsigned long long n)
 {
     return __uint_as_float(S.vstate[(uint32_t)((n + 1ull) & 1ull)]) +
-           __uint_as_float(S.vstate[2u + (uint32_t)(n % 3ull)]);
+           __uint_as_float(S.vstate[2u + mod3(n)]);
+}
+
+// Whether a listed neighbour of a bead at r may lie across a periodic
+// boundary.  Warps without such a bead (97 % of them in a box of 1,400) skip
+// the minimum image of their pairs, six of about 24 instructions each; it
+// would shift by zero, so the forces are the same to the bit.
+template <int D>
+__device__ __forceinline__ bool near_edge(const DevParams& P, float3 r)
+{
+    const bool in = r.x > P.vl_lo[0] && r.x < P.vl_hi[0] && r.y > P.vl_lo[1] && r.y < P.vl_hi[1] &&
+                    (D == 2 || (r.z > P.vl_lo[2] && r.z < P.vl_hi[2]));
+    return !in;
 }
 
 // Verlet pair force: the bead's list from the last build, each pair still
@@ -223,7 +237,7 @@ __device__ __forceinline__ float vl_bound(const StepBuffers& S, unsigned long lo
 // gathers only x and y (8 bytes each, so the batch fits the register budget).
 // A batch's pairs are evaluated without branches, a pair beyond the cut-off
 // (or past the end of the list, fetched as bead i itself) adding 0 * dr.
-template <int D>
+template <int D, bool kWrap>
 __device__ __forceinline__ float3 verlet_force(const DevParams& P, const StepBuffers& S,
                                                const float4* __restrict__ pos, uint32_t i, float3 r)
 {
@@ -241,7 +255,7 @@ __device__ __forceinline__ float3 verlet_force(const DevParams& P, const StepBuf
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float3 dr = subv<D>(f3(pj[q]), r);
-            min_image_near<D>(P, dr);
+            if constexpr (kWrap) min_image_near<D>(P, dr);
             const float rr = dotv<D>(dr, dr);
             const bool in = m + q < k && rr <= P.lj_rc2;
             sub_scaled<D>(f, in ? wca_lj(P, rr) : 0.0f, dr);
@@ -271,6 +285,7 @@ __device__ __forceinline__ PlanarHead planar_head(const DevParams& P, const Step
 
 // verlet_force of planar systems: x and y of six neighbours gathered per
 // batch (8 bytes each), the first batch from the head.
+template <bool kWrap>
 __device__ __forceinline__ float3 verlet_force_planar(const DevParams& P, const StepBuffers& S,
                                                       const float4* __restrict__ pos, uint32_t i, float3 r,
                                                       const PlanarHead& h)
@@ -294,7 +309,7 @@ __device__ __forceinline__ float3 verlet_force_planar(const DevParams& P, const 
 #pragma unroll
         for (int q = 0; q < kPlanarBatch; ++q) {
             float3 dr = make_float3(pj[q].x - r.x, pj[q].y - r.y, 0.f);
-            min_image_near<D>(P, dr);
+            if constexpr (kWrap) min_image_near<D>(P, dr);
             const float rr = dotv<D>(dr, dr);
             const bool in = m + q < k && rr <= P.lj_rc2;
             sub_scaled<D>(f, in ? wca_lj(P, rr) : 0.0f, dr);
@@ -351,9 +366,10 @@ constexpr uint32_t kVlFilled = 6;
 __device__ __forceinline__ void vl_commit(const StepBuffers& S, unsigned long long n, bool rebuilt, float bound)
 {
     S.vstate[(uint32_t)(n & 1ull)] = __float_as_uint(rebuilt ? 0.0f : bound);
-    S.vstate[2u + (uint32_t)((n + 2ull) % 3ull)] = 0u;
-    uint32_t filled = S.vstate[kVlFilled] & ~(1u << (uint32_t)((n + 1ull) % 3ull));
-    if (rebuilt) filled |= 1u << (uint32_t)(n % 3ull);
+    const uint32_t n3 = mod3(n), n4 = n3 == 2u ? 0u : n3 + 1u;
+    S.vstate[2u + (n3 == 0u ? 2u : n3 - 1u)] = 0u;
+    uint32_t filled = S.vstate[kVlFilled] & ~(1u << n4);
+    if (rebuilt) filled |= 1u << n3;
     S.vstate[kVlFilled] = filled;
 }
 
@@ -364,14 +380,17 @@ __device__ __forceinline__ void vl_commit(const StepBuffers& S, unsigned long lo
 // batch kernel, whose parameter block is read from shared memory and whose
 // registers are tighter) keeps the four-wide loop: the batch measured 1 %
 // faster with it, the single system 1.5 % slower.
-template <int CAP, bool kRef, int D, bool kWide = true>
+// kPacked: the update's state is packed (x and y come first in either form).
+template <int CAP, bool kRef, int D, bool kWide = true, bool kPacked = false>
 __device__ __forceinline__ float3 list_pair_force(const DevParams& P, const StepBuffers& S, unsigned long long n,
                                                   uint32_t i, uint32_t blk)
 {
     const uint32_t cur = (uint32_t)(n & 1ull);
-    const uint32_t* cnt = pick3(S.lcount, (uint32_t)(n % 3ull));
+    const uint32_t* cnt = pick3(S.lcount, mod3(n));
     const uint32_t* slots = pick2(S.lslot, cur);
-    const float3 r = f3(pick2(S.pos2, cur)[i]);
+    const float4* __restrict__ pos = kPacked ? pick2(S.pk, cur) : pick2(S.pos2, cur);
+    float3 r = f3(pos[i]);
+    if constexpr (kPacked) r.z = 0.f;
     if (kRef) return ref_list_force<CAP>(P, pick2(S.pos2, cur), pick2(S.vel2, cur), pick2(S.tan2, cur), cnt, slots, i, r);
     if (P.vl_on) {
         PlanarHead head{};
@@ -380,12 +399,16 @@ __device__ __forceinline__ float3 list_pair_force(const DevParams& P, const Step
         const bool rebuild = !(bound <= P.vl_half_skin);  // a NaN bound rebuilds too
         if (blk == 0 && threadIdx.x == 0) vl_commit(S, n, rebuild, bound);
         if (!rebuild) {
-            if constexpr (D == 2 && kWide) return verlet_force_planar(P, S, pick2(S.pos2, cur), i, r, head);
-            else return verlet_force<D>(P, S, pick2(S.pos2, cur), i, r);
+            const bool wrap = __any_sync(__activemask(), near_edge<D>(P, r));
+            if constexpr (D == 2 && kWide)
+                return wrap ? verlet_force_planar<true>(P, S, pos, i, r, head)
+                            : verlet_force_planar<false>(P, S, pos, i, r, head);
+            else
+                return wrap ? verlet_force<D, true>(P, S, pos, i, r) : verlet_force<D, false>(P, S, pos, i, r);
         }
-        return verlet_build_force<CAP, D>(P, S, pick2(S.pos2, cur), cnt, slots, i, r, pick2(S.hash2, cur)[i]);
+        return verlet_build_force<CAP, D>(P, S, pos, cnt, slots, i, r, pick2(S.hash2, cur)[i]);
     }
-    return wca_list_force<CAP, D>(P, pick2(S.pos2, cur), cnt, slots, i, r, pick2(S.hash2, cur)[i]);
+    return wca_list_force<CAP, D>(P, pos, cnt, slots, i, r, pick2(S.hash2, cur)[i]);
 }
 
 // Resident blocks of 256 threads per SM that the WCA fused kernel is
@@ -403,11 +426,14 @@ __host__ __device__ __forceinline__ size_t pro_smem(uint32_t beads, bool reverse
 // pro(n) for the block's filaments: every thread of the block must call it.
 // fprev = F_{n-1} of this thread's bead (complete force of the previous update);
 // blk / nblk = the block's index among, and the number of, its system's blocks.
-// D = 2: a planar WCA system (z carried, forces in the plane).
-template <int CAP, int D>
+// D = 2: a planar WCA system (z carried, forces in the plane).  kPacked:
+// kPackedIn | kPackedOut; with kPackedIn, fold is F_{n-2} of this thread's bead
+// and `from` the buffer that z, radius and mass are taken from.
+template <int CAP, int D, uint32_t kPacked = 0u>
 __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& S, unsigned long long n, float dt,
                                          uint32_t fpb, bool active, uint32_t i, float3 fprev, uint32_t blk,
-                                         uint32_t nblk, bool insert = true, uint32_t pflags = 0u)
+                                         uint32_t nblk, bool insert = true, uint32_t pflags = 0u,
+                                         float2 fold = make_float2(0.f, 0.f), uint32_t from = 0u)
 {
     extern __shared__ float4 sm[];
     const uint32_t L = P.L;
@@ -415,6 +441,7 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     const uint32_t t = threadIdx.x;
     const uint32_t w0 = blk * fpb;
     const uint32_t in = (uint32_t)((n + 1ull) & 1ull), out = (uint32_t)(n & 1ull);
+    const uint32_t n3 = mod3(n);
     float4* smp = sm;                                       // positions [beads]
     float4* smx = sm + (P.reverse_on ? 3u : 1u) * beads;    // triple forces [3][beads]
 
@@ -422,7 +449,7 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     // (Verlet systems fill them only for a rebuild: clear a buffer only when
     // a build filled it since it was last cleared)
     {
-        const uint32_t b = (uint32_t)((n + 1ull) % 3ull);
+        const uint32_t b = n3 == 2u ? 0u : n3 + 1u;
         if (!P.vl_on || ((S.vstate[kVlFilled] >> b) & 1u)) {
             uint32_t* nxt = pick3(S.lcount, b);
             const uint32_t stride = nblk * blockDim.x;
@@ -433,7 +460,25 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     float4 nP = make_float4(0.f, 0.f, 0.f, 0.f), nV = nP, nFo = nP;
     float disp2 = 0.f;  // squared displacement of this update (Verlet list bound)
     if (active) {
-        const float4 P4 = pick2(S.pos2, in)[i], V4 = pick2(S.vel2, in)[i], Fo4 = S.force_old[i];
+        float4 P4 = make_float4(0.f, 0.f, 0.f, 0.f), V4 = P4, Fo4 = P4;
+        if constexpr (kPacked & kPackedIn) {
+            if constexpr (!(kPacked & kPackedOut)) {
+                P4 = pick2(S.pos2, from)[i];
+                V4 = pick2(S.vel2, from)[i];
+                Fo4.w = S.force_old[i].w;
+            }
+            const float4 q = pick2(S.pk, in)[i];
+            P4.x = q.x;
+            P4.y = q.y;
+            V4.x = q.z;
+            V4.y = q.w;
+            Fo4.x = fold.x;
+            Fo4.y = fold.y;
+        } else {
+            P4 = pick2(S.pos2, in)[i];
+            V4 = pick2(S.vel2, in)[i];
+            Fo4 = S.force_old[i];
+        }
         float3 p = f3(P4), v = f3(V4);
         const float3 f = fprev, fo = f3(Fo4);
         // velocity Verlet (particles_kernel_impl.cuh:93-97), per axis:
@@ -488,9 +533,9 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     if (P.vl_on && t == 0) {
         uint32_t m = 0u;
         for (uint32_t q = 0; q < (blockDim.x + 31u) >> 5; ++q) m = s_dmax[q] > m ? s_dmax[q] : m;
-        if (m) atomicMax(&S.vstate[2u + (uint32_t)(n % 3ull)], __float_as_uint(sqrtf(__uint_as_float(m))));
+        if (m) atomicMax(&S.vstate[2u + n3], __float_as_uint(sqrtf(__uint_as_float(m))));
     }
-    const uint32_t wl = active ? t / L : 0u, c = active ? t - wl * L : 0u;
+    const uint32_t wl = active ? fast_div(t, P.L_m, P.L_k) : 0u, c = active ? t - wl * L : 0u;
     const float4* R = smp + wl * L;
     // each bending triple once, by the thread of its first bead
     if (active && L >= 3 && c + 2 < L) {
@@ -545,17 +590,22 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
         if (c > 0) wca_bond<D>(P, me, f3(R[c - 1]), fs);
         if (c + 1 < L) wca_bond_drive<D>(P, me, f3(R[c + 1]), fs);
     }
-    pick2(S.pos2, out)[i] = nP;
-    pick2(S.vel2, out)[i] = nV;
-    S.force_old[i] = nFo;
-    S.force[i] = make_float4(fs.x, fs.y, fs.z, 0.f);
+    if constexpr (kPacked & kPackedOut) {
+        pick2(S.pk, out)[i] = make_float4(nP.x, nP.y, nV.x, nV.y);
+        S.pf[i] = make_float4(fs.x, fs.y, nFo.x, nFo.y);
+    } else {
+        pick2(S.pos2, out)[i] = nP;
+        pick2(S.vel2, out)[i] = nV;
+        S.force_old[i] = nFo;
+        S.force[i] = make_float4(fs.x, fs.y, fs.z, 0.f);
+    }
     if (eager_tan) pick2(S.tan2, out)[i] = wt ? make_float4(tg.x, tg.y, tg.z, 0.f) : pick2(S.tan2, in)[i];
     if (!finitev<D>(f3(nP)) || !finitev<D>(fs)) atomicOr(S.err, (uint32_t)NW_EFLAG_NONFINITE);
 
     if (!insert) return;  // Verlet systems: bead_list_kernel fills list n when a rebuild needs it
     const uint32_t h = P.vl_on ? list_hash(P, f3(nP)) : bead_hash(P, f3(nP));
     pick2(S.hash2, out)[i] = h;
-    const uint32_t slot = atomicAdd(&pick3(S.lcount, (uint32_t)(n % 3ull))[h], 1u);
+    const uint32_t slot = atomicAdd(&pick3(S.lcount, n3)[h], 1u);
     if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = i;
     else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
 }
@@ -565,15 +615,16 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
 // the same words (the displacement bound after update n), so the two always
 // agree.  Otherwise every block leaves after reading the bound.
 template <int CAP>
-__global__ void __launch_bounds__(256) bead_list_kernel(const DevParams P, const StepBuffers S, uint32_t off)
+__global__ void __launch_bounds__(256) bead_list_kernel(const DevParams P, const StepBuffers S, uint32_t off,
+                                                        bool packed)
 {
     pdl_enter();
     const unsigned long long n = *S.step_base + off;
     if (vl_bound(S, n) <= P.vl_half_skin) return;
     const uint32_t out = (uint32_t)(n & 1ull);
-    const float4* __restrict__ pos = pick2(S.pos2, out);
+    const float4* __restrict__ pos = packed ? pick2(S.pk, out) : pick2(S.pos2, out);
     uint32_t* hash = pick2(S.hash2, out);
-    uint32_t* cnt = pick3(S.lcount, (uint32_t)(n % 3ull));
+    uint32_t* cnt = pick3(S.lcount, mod3(n));
     uint32_t* slots = pick2(S.lslot, out);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nb; i += gridDim.x * blockDim.x) {
         const uint32_t h = list_hash(P, f3(pos[i]));
@@ -584,7 +635,7 @@ __global__ void __launch_bounds__(256) bead_list_kernel(const DevParams P, const
     }
 }
 
-template <int CAP, int MAXT, int D>
+template <int CAP, int MAXT, int D, uint32_t kPacked = 0u>
 __global__ void __launch_bounds__(MAXT) bead_pro_kernel(const DevParams P, const StepBuffers S, uint32_t off, float dt,
                                                         uint32_t fpb, uint32_t pflags)
 {
@@ -593,7 +644,7 @@ __global__ void __launch_bounds__(MAXT) bead_pro_kernel(const DevParams P, const
     const uint32_t i = blockIdx.x * fpb * P.L + threadIdx.x;
     const bool active = threadIdx.x < fpb * P.L && i < P.nb;
     const float3 fprev = active ? f3(S.force[i]) : zero3();
-    pro_part<CAP, D>(P, S, n, dt, fpb, active, i, fprev, blockIdx.x, gridDim.x, !P.vl_on, pflags);
+    pro_part<CAP, D, kPacked>(P, S, n, dt, fpb, active, i, fprev, blockIdx.x, gridDim.x, !P.vl_on, pflags);
 }
 
 template <int CAP, bool kRef, int D>
@@ -613,27 +664,31 @@ __global__ void __launch_bounds__(256) bead_epi_kernel(const DevParams P, const 
 }
 
 // epi(n) then pro(n+1): the complete force of update n stays in a register.
-template <int CAP, bool kRef, int MAXT, int D>
+template <int CAP, bool kRef, int MAXT, int D, uint32_t kPacked = 0u>
 __global__ void __launch_bounds__(MAXT, (MAXT == 256 && !kRef) ? NW_FUSED_MIN_BLOCKS : 1)
-    bead_fused_kernel(const DevParams P, const StepBuffers S, uint32_t off, float dt, uint32_t fpb, uint32_t pflags)
+    bead_fused_kernel(const DevParams P, const StepBuffers S, uint32_t off, float dt, uint32_t fpb, uint32_t pflags,
+                      uint32_t from)
 {
     pdl_enter();
-    const unsigned long long n = *S.step_base + off;
+    const unsigned long long base = *S.step_base, n = base + off;
     const uint32_t i = blockIdx.x * fpb * P.L + threadIdx.x;
     const bool active = threadIdx.x < fpb * P.L && i < P.nb;
     float3 Fn = zero3();
+    float2 fold = make_float2(0.f, 0.f);
     if (active) {
-        const float3 pair = list_pair_force<CAP, kRef, D>(P, S, n, i, blockIdx.x);
-        const float4 F = S.force[i];
+        const float3 pair = list_pair_force<CAP, kRef, D, true, (kPacked & kPackedIn) != 0u>(P, S, n, i, blockIdx.x);
+        const float4 F = kPacked & kPackedIn ? S.pf[i] : S.force[i];
+        if constexpr (kPacked & kPackedIn) fold = make_float2(F.z, F.w);
         Fn = make_float3(F.x + pair.x, F.y + pair.y, D == 3 ? F.z + pair.z : 0.f);
         if (!finitev<D>(Fn)) atomicOr(S.err, (uint32_t)NW_EFLAG_NONFINITE);
     }
-    pro_part<CAP, D>(P, S, n + 1ull, dt, fpb, active, i, Fn, blockIdx.x, gridDim.x, !P.vl_on, pflags);
+    pro_part<CAP, D, kPacked>(P, S, n + 1ull, dt, fpb, active, i, Fn, blockIdx.x, gridDim.x, !P.vl_on, pflags, fold,
+                              (uint32_t)(base + from) & 1u);
 }
 
 // A batch block: copy its replica's parameter block into shared memory and
 // run pro, epi or fused for that replica's slice of the batch buffers.
-template <int CAP, int MODE, int MAXT, int D>
+template <int CAP, int MODE, int MAXT, int D, uint32_t kPacked>
 __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const ReplicaSlot* __restrict__ table,
                                                      const uint32_t* __restrict__ block_rep, const StepBuffers S0,
                                                      uint32_t off)
@@ -649,7 +704,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
         const unsigned long long n0 = *S0.step_base + off;
         const uint32_t* vs = S0.vstate + 8u * r;
         const float bound = __uint_as_float(vs[(uint32_t)((n0 + 1ull) & 1ull)]) +
-                            __uint_as_float(vs[2u + (uint32_t)(n0 % 3ull)]);
+                            __uint_as_float(vs[2u + mod3(n0)]);
         if (!e->P.vl_on || bound <= e->P.vl_half_skin) return;
     }
     {
@@ -672,6 +727,11 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
     for (int k = 0; k < 3; ++k) S.lcount[k] += co;
     S.force += bo;
     S.force_old += bo;
+    if constexpr (kPacked != 0u) {
+        S.pk[0] += bo;
+        S.pk[1] += bo;
+        S.pf += bo;
+    }
     if (S.nbr) S.nbr += e->nbr_off;
     if (S.nnb) S.nnb += bo;
     if (S.vstate) S.vstate += 8u * r;
@@ -682,27 +742,32 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
         // this replica's cell list of update n, only when its pair pass rebuilds
         if (!P.vl_on || vl_bound(S, n) <= P.vl_half_skin || !active) return;
         const uint32_t out = (uint32_t)(n & 1ull);
-        const uint32_t h = list_hash(P, f3(pick2(S.pos2, out)[i]));
+        const uint32_t h = list_hash(P, f3((kPacked ? pick2(S.pk, out) : pick2(S.pos2, out))[i]));
         pick2(S.hash2, out)[i] = h;
-        const uint32_t slot = atomicAdd(&pick3(S.lcount, (uint32_t)(n % 3ull))[h], 1u);
+        const uint32_t slot = atomicAdd(&pick3(S.lcount, mod3(n))[h], 1u);
         if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = i;
         else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
         return;
     }
     if (MODE == kBatchPro) {
         const float3 fprev = active ? f3(S.force[i]) : zero3();
-        pro_part<CAP, D>(P, S, n, dt, fpb, active, i, fprev, blk, nblk, !P.vl_on, pro_flags(P));
+        pro_part<CAP, D, kPacked>(P, S, n, dt, fpb, active, i, fprev, blk, nblk, !P.vl_on, pro_flags(P));
         return;
     }
     float3 Fn = zero3();
+    float2 fold = make_float2(0.f, 0.f);
     if (active) {
-        const float3 pair = list_pair_force<CAP, false, D, false>(P, S, n, i, blk);
-        const float4 F = S.force[i];
-        Fn = make_float3(F.x + pair.x, F.y + pair.y, D == 3 ? F.z + pair.z : F.z);
+        const float3 pair = list_pair_force<CAP, false, D, false, (kPacked & kPackedIn) != 0u>(P, S, n, i, blk);
+        const float4 F = kPacked & kPackedIn ? S.pf[i] : S.force[i];
+        if constexpr (kPacked & kPackedIn) fold = make_float2(F.z, F.w);
+        Fn = make_float3(F.x + pair.x, F.y + pair.y, D == 3 ? F.z + pair.z : (kPacked & kPackedIn ? 0.f : F.z));
         if (!finitev<D>(Fn)) atomicOr(S.err, (uint32_t)NW_EFLAG_NONFINITE);
         if (MODE == kBatchEpi) S.force[i] = make_float4(Fn.x, Fn.y, Fn.z, F.w);
     }
-    if (MODE == kBatchFused) pro_part<CAP, D>(P, S, n + 1ull, dt, fpb, active, i, Fn, blk, nblk, !P.vl_on, pro_flags(P));
+    // a packed call left the API's arrays before its first update
+    if (MODE == kBatchFused)
+        pro_part<CAP, D, kPacked>(P, S, n + 1ull, dt, fpb, active, i, Fn, blk, nblk, !P.vl_on, pro_flags(P), fold,
+                                  (uint32_t)(*S.step_base + 1ull) & 1u);
 }
 
 // Bead tangents of the current positions, as the pro part writes them
@@ -734,7 +799,7 @@ inline void pro_shape(const DevParams& P, uint32_t& fpb, uint32_t& threads, size
 // ---- launchers of one dimension (D = 3, or 2 for planar systems) ------------
 
 template <int D>
-uint64_t bead_pro_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s)
+uint64_t bead_pro_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed, cudaStream_t s)
 {
     uint32_t fpb, threads;
     size_t smem;
@@ -742,6 +807,14 @@ uint64_t bead_pro_d(const DevParams& P, const StepBuffers& B, uint32_t off, floa
     const uint32_t blocks = cdiv32(P.nf, fpb);
     const bool big = threads > 256;  // filaments longer than 256 beads: one per block, up to 1024 threads
     const uint32_t pf = pro_flags(P);
+    if constexpr (D == 2) {
+        if (packed & kPackedOut) {
+            if (B.cap == 16)
+                launch_pdl(bead_pro_kernel<16, 256, 2, kPackedOut>, blocks, threads, smem, s, P, B, off, dt, fpb, pf);
+            else launch_pdl(bead_pro_kernel<8, 256, 2, kPackedOut>, blocks, threads, smem, s, P, B, off, dt, fpb, pf);
+            return 1;
+        }
+    }
     if (B.cap == 16) {
         if (big) launch_pdl(bead_pro_kernel<16, 1024, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf);
         else launch_pdl(bead_pro_kernel<16, 256, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf);
@@ -778,7 +851,8 @@ uint64_t bead_epi_d(const DevParams& P, const StepBuffers& B, uint32_t off, cuda
 }
 
 template <int D>
-uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s)
+uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed, uint32_t from,
+                      cudaStream_t s)
 {
     uint32_t fpb, threads;
     size_t smem;
@@ -789,9 +863,24 @@ uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, fl
     const uint32_t pf = pro_flags(P);
 #define NW_FUSED(CAPV, REFV)                                                                                   \
     do {                                                                                                       \
-        if (big) launch_pdl(bead_fused_kernel<CAPV, REFV, 1024, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf); \
-        else launch_pdl(bead_fused_kernel<CAPV, REFV, 256, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf);      \
+        if (big) launch_pdl(bead_fused_kernel<CAPV, REFV, 1024, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf, from); \
+        else launch_pdl(bead_fused_kernel<CAPV, REFV, 256, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf, from);      \
     } while (0)
+    if constexpr (D == 2) {
+#define NW_FUSED_PACKED(CAPV)                                                                                      \
+    do {                                                                                                           \
+        auto* k = packed == (kPackedIn | kPackedOut) ? bead_fused_kernel<CAPV, false, 256, 2, kPackedIn | kPackedOut> \
+                  : packed == kPackedIn              ? bead_fused_kernel<CAPV, false, 256, 2, kPackedIn>              \
+                                                     : bead_fused_kernel<CAPV, false, 256, 2, kPackedOut>;            \
+        launch_pdl(k, blocks, threads, smem, s, P, B, off, dt, fpb, pf, from);                                     \
+    } while (0)
+        if (packed) {
+            if (B.cap == 16) NW_FUSED_PACKED(16);
+            else NW_FUSED_PACKED(8);
+            return 1;
+        }
+#undef NW_FUSED_PACKED
+    }
     if constexpr (D == 3) {
         if (ref) {
             if (B.cap == 16) NW_FUSED(16, true);
@@ -807,25 +896,41 @@ uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, fl
 
 template <int D>
 void batch_d(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks, uint32_t threads,
-             size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off, cudaStream_t s)
+             size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off, uint32_t packed, cudaStream_t s)
 {
     const bool big = threads > 256;
-#define NW_BATCH(CAPV, MODEV)                                                                                    \
-    do {                                                                                                         \
-        if (big) batch_kernel<CAPV, MODEV, 512, D><<<blocks, threads, smem, s>>>(table, block_rep, S, off);     \
-        else batch_kernel<CAPV, MODEV, 256, D><<<blocks, threads, smem, s>>>(table, block_rep, S, off);         \
-    } while (0)
-#define NW_BATCH_MODE(CAPV)                                      \
-    do {                                                         \
-        if (mode == kBatchPro) NW_BATCH(CAPV, kBatchPro);        \
-        else if (mode == kBatchEpi) NW_BATCH(CAPV, kBatchEpi);   \
-        else if (mode == kBatchList) NW_BATCH(CAPV, kBatchList); \
-        else NW_BATCH(CAPV, kBatchFused);                        \
-    } while (0)
-    if (cap == 16) NW_BATCH_MODE(16);
-    else NW_BATCH_MODE(8);
-#undef NW_BATCH_MODE
-#undef NW_BATCH
+    auto go = [&](auto cap_c, auto mode_c, auto packed_c) {
+        constexpr int C = decltype(cap_c)::value, M = decltype(mode_c)::value;
+        constexpr uint32_t K = decltype(packed_c)::value;
+        if (big) batch_kernel<C, M, 512, D, K><<<blocks, threads, smem, s>>>(table, block_rep, S, off);
+        else batch_kernel<C, M, 256, D, K><<<blocks, threads, smem, s>>>(table, block_rep, S, off);
+    };
+    auto of_mode = [&](auto cap_c, auto packed_c) {
+        // forms that occur: the list kernel reads either, pro only writes packed,
+        // epi reads the API's arrays
+        constexpr uint32_t K = decltype(packed_c)::value;
+        if constexpr (K == 0u || K == kPackedOut) {
+            if (mode == kBatchPro) return go(cap_c, std::integral_constant<int, kBatchPro>{}, packed_c);
+        }
+        if constexpr (K == 0u) {
+            if (mode == kBatchEpi) return go(cap_c, std::integral_constant<int, kBatchEpi>{}, packed_c);
+        }
+        if constexpr (K == 0u || K == kPackedIn) {
+            if (mode == kBatchList) return go(cap_c, std::integral_constant<int, kBatchList>{}, packed_c);
+        }
+        if (mode == kBatchFused) go(cap_c, std::integral_constant<int, kBatchFused>{}, packed_c);
+    };
+    auto of_packed = [&](auto cap_c) {
+        if constexpr (D == 2) {
+            if (packed == (kPackedIn | kPackedOut))
+                return of_mode(cap_c, std::integral_constant<uint32_t, kPackedIn | kPackedOut>{});
+            if (packed == kPackedIn) return of_mode(cap_c, std::integral_constant<uint32_t, kPackedIn>{});
+            if (packed == kPackedOut) return of_mode(cap_c, std::integral_constant<uint32_t, kPackedOut>{});
+        }
+        of_mode(cap_c, std::integral_constant<uint32_t, 0u>{});
+    };
+    if (cap == 16) of_packed(std::integral_constant<int, 16>{});
+    else of_packed(std::integral_constant<int, 8>{});
 }
 
 }  // namespace

@@ -5,9 +5,10 @@
 
 namespace nw {
 
-uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s)
+uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                                cudaStream_t s)
 {
-    return bead_pro_d<2>(P, B, off, dt, s);
+    return bead_pro_d<2>(P, B, off, dt, packed, s);
 }
 
 uint64_t launch_bead_tangents_planar(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s)
@@ -20,16 +21,17 @@ uint64_t launch_bead_epi_planar(const DevParams& P, const StepBuffers& B, uint32
     return bead_epi_d<2>(P, B, off, s);
 }
 
-uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, cudaStream_t s)
+uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
+                                  uint32_t from, cudaStream_t s)
 {
-    return bead_fused_d<2>(P, B, off, dt, s);
+    return bead_fused_d<2>(P, B, off, dt, packed, from, s);
 }
 
 void launch_batch_planar(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks,
                          uint32_t threads, size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off,
-                         cudaStream_t s)
+                         uint32_t packed, cudaStream_t s)
 {
-    batch_d<2>(mode, table, block_rep, blocks, threads, smem, cap, S, off, s);
+    batch_d<2>(mode, table, block_rep, blocks, threads, smem, cap, S, off, packed, s);
 }
 
 }  // namespace nw

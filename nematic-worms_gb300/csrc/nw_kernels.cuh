@@ -74,6 +74,10 @@ struct StepBuffers {
     // the sorted path updates in place, with both entries naming one array.
     float4 *pos2[2], *vel2[2], *tan2[2];
     uint32_t* hash2[2];
+    // packed bead state of planar Verlet systems between the updates of one
+    // call (kPackedIn / kPackedOut, nw_fused.cuh): (x, y, v_x, v_y) of update n
+    // in pk[n & 1], (partial force x, y, previous force x, y) in pf
+    float4 *pk[2], *pf;
     // in-place views of the sorted path (= pos2[0], ...)
     float4 *pos, *vel, *force, *force_old, *tangent;
     uint32_t *hash, *slot, *tmp_index, *sorted_index, *sorted_hash;
