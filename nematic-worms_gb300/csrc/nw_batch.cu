@@ -264,7 +264,8 @@ uint64_t enqueue(nw_batch* b, int nsteps)
     if (b->blocks == 0) return 0;
     uint64_t launches = 0;
     auto L = [&](int mode, uint32_t off, uint32_t packed) {
-        launch_batch(mode, b->d_slots, b->d_block_rep, b->blocks, b->threads, b->smem, b->cap, b->B, off, b->planar,
+        const uint32_t blocks = mode == kBatchList ? (uint32_t)b->R * kBatchListBlocks : b->blocks;
+        launch_batch(mode, b->d_slots, b->d_block_rep, blocks, b->threads, b->smem, b->cap, b->B, off, b->planar,
                      packed, b->stream);
         ++launches;
     };
@@ -281,7 +282,7 @@ uint64_t enqueue(nw_batch* b, int nsteps)
             if (b->vl) L(kBatchList, (uint32_t)(j + 1), in(j + 1));
         }
     }
-    advance_step_kernel<<<1, 1, 0, b->stream>>>(b->B.step_base, (unsigned long long)nsteps);
+    launch_pdl(advance_step_kernel, 1, 1, 0, b->stream, b->B.step_base, (unsigned long long)nsteps);
     return launches + 1ull;
 }
 

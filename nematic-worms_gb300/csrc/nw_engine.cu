@@ -381,10 +381,11 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
         // updates that leave their state packed: neither read by a collision nor the last
         const bool pack = packs(P) && s->B.pf;  // no packed buffers where reversal was switched off later
         auto packed = [&](int j) { return pack && j < nsteps - 1 && !hit(j); };
+        const uint32_t insert = inserts(P, nsteps) ? kProInsert : 0u;
         uint32_t from = 1u;  // parity of the last update in the API's arrays (-1: the state before the call)
         auto list = [&](int j) {
             if (!packed(j)) from = (uint32_t)j & 1u;
-            if (!P.vl_on) return;
+            if (!P.vl_on || insert) return;
             NW_MARK("bead_list");
             launches += launch_bead_list(P, s->B, (uint32_t)j, packed(j), s->stream);
         };
@@ -393,7 +394,7 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
                                     prof, 2u);
         };
         NW_MARK("bead_pro");
-        launches += launch_bead_pro(P, s->B, 0u, dt, packed(0) ? kPackedOut : 0u, s->stream);
+        launches += launch_bead_pro(P, s->B, 0u, dt, packed(0) ? kPackedOut : 0u, insert, s->stream);
         list(0);
         for (int j = 0; j < nsteps; ++j) {
             const bool srd_now = hit(j);
@@ -406,14 +407,14 @@ uint64_t enqueue_steps(nw_system* s, int nsteps, float dt, uint64_t first_step, 
                 if (srd_now && !wca) collide((uint32_t)j);
                 if (j < nsteps - 1) {
                     NW_MARK("bead_pro");
-                    launches += launch_bead_pro(P, s->B, (uint32_t)(j + 1), dt, 0u, s->stream);
+                    launches += launch_bead_pro(P, s->B, (uint32_t)(j + 1), dt, 0u, 0u, s->stream);
                     list(j + 1);
                 }
             } else {
                 NW_MARK("bead_fused");
                 launches += launch_bead_fused(P, s->B, (uint32_t)j, dt,
                                               (packed(j) ? kPackedIn : 0u) | (packed(j + 1) ? kPackedOut : 0u), from,
-                                              s->stream);
+                                              insert, s->stream);
                 list(j + 1);
             }
         }

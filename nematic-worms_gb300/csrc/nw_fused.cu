@@ -13,10 +13,11 @@ uint32_t list_filaments_per_block(uint32_t L, uint32_t nf)
 }
 
 uint64_t launch_bead_pro(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                         cudaStream_t s)
+                         uint32_t insert, cudaStream_t s)
 {
     if (P.nb == 0) return 0;
-    return planar_system(P) ? launch_bead_pro_planar(P, B, off, dt, packed, s) : bead_pro_d<3>(P, B, off, dt, 0u, s);
+    return planar_system(P) ? launch_bead_pro_planar(P, B, off, dt, packed, insert, s)
+                            : bead_pro_d<3>(P, B, off, dt, 0u, insert, s);
 }
 
 uint64_t launch_bead_tangents(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s)
@@ -41,11 +42,11 @@ uint64_t launch_bead_epi(const DevParams& P, const StepBuffers& B, uint32_t off,
 }
 
 uint64_t launch_bead_fused(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                           uint32_t from, cudaStream_t s)
+                           uint32_t from, uint32_t insert, cudaStream_t s)
 {
     if (P.nb == 0) return 0;
-    return planar_system(P) ? launch_bead_fused_planar(P, B, off, dt, packed, from, s)
-                            : bead_fused_d<3>(P, B, off, dt, 0u, from, s);
+    return planar_system(P) ? launch_bead_fused_planar(P, B, off, dt, packed, from, insert, s)
+                            : bead_fused_d<3>(P, B, off, dt, 0u, from, insert, s);
 }
 
 void launch_batch(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks, uint32_t threads,

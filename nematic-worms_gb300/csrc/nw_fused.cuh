@@ -10,11 +10,25 @@ namespace nw {
 //   kProLazyTangent  tangents are not stored by the step (WCA worms of more
 //                    than three beads, whose step never reads them); the
 //                    handle API computes them when they are read
-constexpr uint32_t kProLazyTangent = 1u;
+//   kProInsert       every update's pro part fills its cell list, and no
+//                    bead_list launch follows (inserts())
+constexpr uint32_t kProLazyTangent = 1u, kProInsert = 2u;
 __host__ __device__ __forceinline__ uint32_t pro_flags(const DevParams& P)
 {
     return P.model == NW_MODEL_WCA_WORMS && P.L > 3u ? kProLazyTangent : 0u;
 }
+// Small Verlet systems fill every update's cell list in the pro part, although
+// only list builds read it: the atomics and the clearing cost less than a
+// launch that mostly leaves at once (about 1.2 us).  At 400,000 beads they cost
+// 0.9 us more than it, so the line lies at a third of that; 100 updates of
+// 4,000 beads (three such systems at a time) take 224 us so, and 230 with the
+// launch; alone 581 and 680.  Calls of one update keep the launch.
+constexpr uint32_t kInsertBeads = 131072;
+__host__ __device__ __forceinline__ bool inserts(const DevParams& P, int nsteps)
+{
+    return P.vl_on && nsteps > 1 && P.nb <= kInsertBeads;
+}
+
 // Within one call, the bead state of planar Verlet systems between updates is
 // packed: two float4 a bead (x, y, velocity; partial and previous force)
 // instead of four, since z, the radius and the mass stay as they are and the
@@ -38,8 +52,9 @@ uint32_t list_filaments_per_block(uint32_t L, uint32_t nf);
 
 // pro(n) with n = *step_base + off: integrate .. hash, insert into list n.
 // packed: kPackedOut or 0.
+// insert: kProInsert or 0.
 uint64_t launch_bead_pro(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                         cudaStream_t s);
+                         uint32_t insert, cudaStream_t s);
 // Verlet systems: the cell list of update n, built only when the pair pass
 // of update n rebuilds the neighbour lists (launch after the pro part of n).
 // packed: whether update n left its state packed.
@@ -50,7 +65,7 @@ uint64_t launch_bead_epi(const DevParams& P, const StepBuffers& B, uint32_t off,
 // from: parity of the offset of the last update in the API's arrays (-1, the
 // state before the call, is odd).
 uint64_t launch_bead_fused(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                           uint32_t from, cudaStream_t s);
+                           uint32_t from, uint32_t insert, cudaStream_t s);
 
 // ---- batched replicas (nw_batch.cu) ------------------------------------------
 
@@ -70,7 +85,9 @@ struct ReplicaSlot {
 };
 
 // kBatchList: a replica's cell list of update n when its pair pass will
-// rebuild the Verlet lists (Verlet replicas; launched after each pro part)
+// rebuild the Verlet lists (Verlet replicas; launched after each pro part);
+// kBatchListBlocks blocks for each replica, which mostly leave at once
+constexpr uint32_t kBatchListBlocks = 8;
 enum BatchMode { kBatchPro = 0, kBatchEpi = 1, kBatchFused = 2, kBatchList = 3 };
 
 // One launch over all replicas: block b serves replica block_rep[b].  S holds
@@ -82,11 +99,11 @@ void launch_batch(int mode, const ReplicaSlot* table, const uint32_t* block_rep,
 
 // The two-component launches (nw_fused_planar.cu) behind the launchers above.
 uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                                cudaStream_t s);
+                                uint32_t insert, cudaStream_t s);
 uint64_t launch_bead_tangents_planar(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s);
 uint64_t launch_bead_epi_planar(const DevParams& P, const StepBuffers& B, uint32_t off, cudaStream_t s);
 uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                                  uint32_t from, cudaStream_t s);
+                                  uint32_t from, uint32_t insert, cudaStream_t s);
 void launch_batch_planar(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks,
                          uint32_t threads, size_t smem, uint32_t cap, const StepBuffers& S, uint32_t off,
                          uint32_t packed, cudaStream_t s);

@@ -329,6 +329,7 @@ __device__ __forceinline__ float3 verlet_build_force(const DevParams& P, const S
                                                      uint32_t own)
 {
     const uint32_t fbase = (i / P.L) * P.L;
+    if (__ldg(cnt + own) > (uint32_t)CAP) atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
     uint32_t k = 0;
     uint32_t* col = S.nbr + i;
     float3 f = zero3();
@@ -446,11 +447,11 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     float4* smx = sm + (P.reverse_on ? 3u : 1u) * beads;    // triple forces [3][beads]
 
     // lists of update n+1 must start empty: clear them while nobody reads them
-    // (Verlet systems fill them only for a rebuild: clear a buffer only when
-    // a build filled it since it was last cleared)
+    // (without insert, Verlet systems fill them only for a rebuild: a buffer is
+    // cleared only when one filled it since it was last cleared)
     {
         const uint32_t b = n3 == 2u ? 0u : n3 + 1u;
-        if (!P.vl_on || ((S.vstate[kVlFilled] >> b) & 1u)) {
+        if (insert || ((S.vstate[kVlFilled] >> b) & 1u)) {
             uint32_t* nxt = pick3(S.lcount, b);
             const uint32_t stride = nblk * blockDim.x;
             for (uint32_t c = blk * blockDim.x + t; c < P.lncells; c += stride) nxt[c] = 0u;
@@ -530,6 +531,8 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     }
     if (active) smp[t] = nP;
     __syncthreads();
+    // the thread that keeps the lists' books (vl_commit)
+    if (P.vl_on && insert && blk == 0 && t == 0) S.vstate[kVlFilled] |= 1u << n3;
     if (P.vl_on && t == 0) {
         uint32_t m = 0u;
         for (uint32_t q = 0; q < (blockDim.x + 31u) >> 5; ++q) m = s_dmax[q] > m ? s_dmax[q] : m;
@@ -607,7 +610,7 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
     pick2(S.hash2, out)[i] = h;
     const uint32_t slot = atomicAdd(&pick3(S.lcount, n3)[h], 1u);
     if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = i;
-    else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
+    else if (!P.vl_on) atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);  // Verlet: when a build reads the list
 }
 
 // The cell list of update n for a Verlet system, built only when the pair
@@ -644,7 +647,7 @@ __global__ void __launch_bounds__(MAXT) bead_pro_kernel(const DevParams P, const
     const uint32_t i = blockIdx.x * fpb * P.L + threadIdx.x;
     const bool active = threadIdx.x < fpb * P.L && i < P.nb;
     const float3 fprev = active ? f3(S.force[i]) : zero3();
-    pro_part<CAP, D, kPacked>(P, S, n, dt, fpb, active, i, fprev, blockIdx.x, gridDim.x, !P.vl_on, pflags);
+    pro_part<CAP, D, kPacked>(P, S, n, dt, fpb, active, i, fprev, blockIdx.x, gridDim.x, !P.vl_on || (pflags & kProInsert), pflags);
 }
 
 template <int CAP, bool kRef, int D>
@@ -682,7 +685,7 @@ __global__ void __launch_bounds__(MAXT, (MAXT == 256 && !kRef) ? NW_FUSED_MIN_BL
         Fn = make_float3(F.x + pair.x, F.y + pair.y, D == 3 ? F.z + pair.z : 0.f);
         if (!finitev<D>(Fn)) atomicOr(S.err, (uint32_t)NW_EFLAG_NONFINITE);
     }
-    pro_part<CAP, D, kPacked>(P, S, n + 1ull, dt, fpb, active, i, Fn, blockIdx.x, gridDim.x, !P.vl_on, pflags, fold,
+    pro_part<CAP, D, kPacked>(P, S, n + 1ull, dt, fpb, active, i, Fn, blockIdx.x, gridDim.x, !P.vl_on || (pflags & kProInsert), pflags, fold,
                               (uint32_t)(base + from) & 1u);
 }
 
@@ -693,8 +696,9 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
                                                      const uint32_t* __restrict__ block_rep, const StepBuffers S0,
                                                      uint32_t off)
 {
+    pdl_enter();
     __shared__ DevParams sP;
-    const uint32_t r = __ldg(block_rep + blockIdx.x);
+    const uint32_t r = MODE == kBatchList ? blockIdx.x / kBatchListBlocks : __ldg(block_rep + blockIdx.x);
     const ReplicaSlot* e = table + r;
     if (MODE == kBatchList) {
         // leave before staging the parameter block unless this replica rebuilds
@@ -740,13 +744,16 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
     const bool active = threadIdx.x < fpb * P.L && i < P.nb;
     if (MODE == kBatchList) {
         // this replica's cell list of update n, only when its pair pass rebuilds
-        if (!P.vl_on || vl_bound(S, n) <= P.vl_half_skin || !active) return;
         const uint32_t out = (uint32_t)(n & 1ull);
-        const uint32_t h = list_hash(P, f3((kPacked ? pick2(S.pk, out) : pick2(S.pos2, out))[i]));
-        pick2(S.hash2, out)[i] = h;
-        const uint32_t slot = atomicAdd(&pick3(S.lcount, mod3(n))[h], 1u);
-        if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = i;
-        else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
+        const float4* __restrict__ pos = kPacked ? pick2(S.pk, out) : pick2(S.pos2, out);
+        for (uint32_t j = (blockIdx.x % kBatchListBlocks) * blockDim.x + threadIdx.x; j < P.nb;
+             j += kBatchListBlocks * blockDim.x) {
+            const uint32_t h = list_hash(P, f3(pos[j]));
+            pick2(S.hash2, out)[j] = h;
+            const uint32_t slot = atomicAdd(&pick3(S.lcount, mod3(n))[h], 1u);
+            if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = j;
+            else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
+        }
         return;
     }
     if (MODE == kBatchPro) {
@@ -799,14 +806,15 @@ inline void pro_shape(const DevParams& P, uint32_t& fpb, uint32_t& threads, size
 // ---- launchers of one dimension (D = 3, or 2 for planar systems) ------------
 
 template <int D>
-uint64_t bead_pro_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed, cudaStream_t s)
+uint64_t bead_pro_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed, uint32_t insert,
+                    cudaStream_t s)
 {
     uint32_t fpb, threads;
     size_t smem;
     pro_shape(P, fpb, threads, smem);
     const uint32_t blocks = cdiv32(P.nf, fpb);
     const bool big = threads > 256;  // filaments longer than 256 beads: one per block, up to 1024 threads
-    const uint32_t pf = pro_flags(P);
+    const uint32_t pf = pro_flags(P) | insert;
     if constexpr (D == 2) {
         if (packed & kPackedOut) {
             if (B.cap == 16)
@@ -852,7 +860,7 @@ uint64_t bead_epi_d(const DevParams& P, const StepBuffers& B, uint32_t off, cuda
 
 template <int D>
 uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed, uint32_t from,
-                      cudaStream_t s)
+                      uint32_t insert, cudaStream_t s)
 {
     uint32_t fpb, threads;
     size_t smem;
@@ -860,7 +868,7 @@ uint64_t bead_fused_d(const DevParams& P, const StepBuffers& B, uint32_t off, fl
     const uint32_t blocks = cdiv32(P.nf, fpb);
     const bool ref = P.model == NW_MODEL_REF_DEM;
     const bool big = threads > 256;
-    const uint32_t pf = pro_flags(P);
+    const uint32_t pf = pro_flags(P) | insert;
 #define NW_FUSED(CAPV, REFV)                                                                                   \
     do {                                                                                                       \
         if (big) launch_pdl(bead_fused_kernel<CAPV, REFV, 1024, D>, blocks, threads, smem, s, P, B, off, dt, fpb, pf, from); \
@@ -902,8 +910,8 @@ void batch_d(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint
     auto go = [&](auto cap_c, auto mode_c, auto packed_c) {
         constexpr int C = decltype(cap_c)::value, M = decltype(mode_c)::value;
         constexpr uint32_t K = decltype(packed_c)::value;
-        if (big) batch_kernel<C, M, 512, D, K><<<blocks, threads, smem, s>>>(table, block_rep, S, off);
-        else batch_kernel<C, M, 256, D, K><<<blocks, threads, smem, s>>>(table, block_rep, S, off);
+        auto* kernel = big ? batch_kernel<C, M, 512, D, K> : batch_kernel<C, M, 256, D, K>;
+        launch_pdl(kernel, blocks, threads, M == kBatchList ? (size_t)0 : smem, s, table, block_rep, S, off);
     };
     auto of_mode = [&](auto cap_c, auto packed_c) {
         // forms that occur: the list kernel reads either, pro only writes packed,

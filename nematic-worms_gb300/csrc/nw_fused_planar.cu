@@ -6,9 +6,9 @@
 namespace nw {
 
 uint64_t launch_bead_pro_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                                cudaStream_t s)
+                                uint32_t insert, cudaStream_t s)
 {
-    return bead_pro_d<2>(P, B, off, dt, packed, s);
+    return bead_pro_d<2>(P, B, off, dt, packed, insert, s);
 }
 
 uint64_t launch_bead_tangents_planar(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s)
@@ -22,9 +22,9 @@ uint64_t launch_bead_epi_planar(const DevParams& P, const StepBuffers& B, uint32
 }
 
 uint64_t launch_bead_fused_planar(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
-                                  uint32_t from, cudaStream_t s)
+                                  uint32_t from, uint32_t insert, cudaStream_t s)
 {
-    return bead_fused_d<2>(P, B, off, dt, packed, from, s);
+    return bead_fused_d<2>(P, B, off, dt, packed, from, insert, s);
 }
 
 void launch_batch_planar(int mode, const ReplicaSlot* table, const uint32_t* block_rep, uint32_t blocks,
