@@ -391,8 +391,9 @@ nw_status nw_batch_create(const NwConfig* replicas, int n, nw_batch** out)
     A(balloc(b->state_allocs, &B.force, nbt));
     A(balloc(b->state_allocs, &B.force_old, nbt));
     if (b->planar) {
-        for (int k = 0; k < 2; ++k) A(balloc(b->state_allocs, &B.pk[k], nbt));
-        A(balloc(b->state_allocs, &B.pf, nbt));
+        A(balloc(b->state_allocs, &B.pk[0], 3 * nbt));  // one allocation: pk[0], pk[1], pf
+        B.pk[1] = B.pk[0] + nbt;
+        B.pf = B.pk[1] + nbt;
     }
     A(balloc(b->state_allocs, &B.err, 4));
     A(balloc(b->state_allocs, &B.step_base, 1));

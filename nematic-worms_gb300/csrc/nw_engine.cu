@@ -208,9 +208,11 @@ __global__ void __launch_bounds__(256) ref_hash_kernel(const DevParams P, const 
 // displacement is taken (non-negative floats order as their bits); the
 // displacement is then added to the lists' bound, so unchanged or slightly
 // moved beads keep their lists and larger moves rebuild them.
+// The last block to finish adds the displacement (vstate[7] counts them).
 __global__ void __launch_bounds__(256) set_positions_kernel(const float4* __restrict__ src, float4* __restrict__ dst,
-                                                            uint32_t n, uint32_t* __restrict__ dmax)
+                                                            uint32_t n, uint32_t* vstate, uint32_t slot)
 {
+    uint32_t* dmax = vstate + 5;
     uint32_t m = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 a = src[i], b = dst[i];
@@ -227,14 +229,13 @@ __global__ void __launch_bounds__(256) set_positions_kernel(const float4* __rest
     if (threadIdx.x == 0) {  // one atomic per block on the shared word
         for (uint32_t q = 1; q < (blockDim.x >> 5); ++q) m = s_m[q] > m ? s_m[q] : m;
         if (m) atomicMax(dmax, m);
+        __threadfence();
+        if (atomicAdd(vstate + 7, 1u) + 1u == gridDim.x) {  // every block's maximum is in
+            const float d = sqrtf(__uint_as_float(atomicExch(dmax, 0u)));
+            vstate[slot] = __float_as_uint(__uint_as_float(vstate[slot]) + d);
+            vstate[7] = 0u;
+        }
     }
-}
-
-__global__ void vl_add_displacement_kernel(uint32_t* __restrict__ vstate, uint32_t slot)
-{
-    const float d = sqrtf(__uint_as_float(vstate[5]));
-    vstate[slot] = __float_as_uint(__uint_as_float(vstate[slot]) + d);
-    vstate[5] = 0u;
 }
 
 }  // namespace nw
@@ -493,6 +494,8 @@ cudaError_t release_solvent_order(nw_system* s)
 
 enum class Dir { ToDevice, ToHost };
 
+constexpr uint32_t kEarlyReadMin = 32768;  // elements of an early read-back (512 KB)
+
 // Copy `count` elements of an API array between host and device.  Position /
 // velocity arrays are beads [0, nb) then solvent [nb, nb + ns) in two stores.
 nw_status transfer(nw_system* s, int array, void* host, uint32_t start, uint32_t count, Dir dir, bool wait = true)
@@ -500,7 +503,10 @@ nw_status transfer(nw_system* s, int array, void* host, uint32_t start, uint32_t
     // an asynchronous read of positions or velocities right after a step
     // starts on aux once they are final (state_ev), beside the step's pair
     // pass; the engine's stream then waits for it
-    const bool early = dir == Dir::ToHost && !wait && s->state_ev_valid &&
+    // (short copies go on the engine's stream: the events and the waits that
+    // an early one takes cost the host more than the pair pass that it would
+    // run beside, about 3 us against 5 for 4,000 beads)
+    const bool early = dir == Dir::ToHost && !wait && s->state_ev_valid && count >= kEarlyReadMin &&
                        (array == NW_POSITION || array == NW_VELOCITY);
     if (dir == Dir::ToDevice) s->state_ev_valid = false;
     cudaStream_t cs = s->stream;
@@ -571,8 +577,8 @@ nw_status transfer(nw_system* s, int array, void* host, uint32_t start, uint32_t
         if (e == cudaSuccess) {
             const uint32_t n = (uint32_t)(b - a);
             const uint32_t blocks = std::min<uint32_t>((n + 255u) / 256u, 4u * 152u);
-            set_positions_kernel<<<blocks, 256, 0, s->stream>>>(stage, B.pos2[cur] + a, n, B.vstate + 5);
-            vl_add_displacement_kernel<<<1, 1, 0, s->stream>>>(B.vstate, (uint32_t)((s->step + 1ull) & 1ull));
+            set_positions_kernel<<<blocks, 256, 0, s->stream>>>(stage, B.pos2[cur] + a, n, B.vstate,
+                                                                (uint32_t)((s->step + 1ull) & 1ull));
             e = cudaGetLastError();
         }
         h += (b - a) * elem;
@@ -707,8 +713,9 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.lslot[k], LC * B.cap + 8));
     }
     if (packs(P0)) {
-        for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.pk[k], nb));
-        A(alloc_n(s, &B.pf, nb));
+        A(alloc_n(s, &B.pk[0], 3 * nb));  // one allocation: pk[0], pk[1], pf
+        B.pk[1] = B.pk[0] + nb;
+        B.pf = B.pk[1] + nb;
     }
     if (s->vl) {
         A(alloc_n(s, &B.nbr, (size_t)P0.vl_cap * nb + 8));
@@ -726,8 +733,8 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         A(alloc_n(s, &B.srd_scount, Cs + 8));
         A(alloc_n(s, &B.srd_boff, Cs + 8));
         for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.srd_soff2[k], Cs + 8));
-        A(alloc_n(s, &B.srd_btab, Cs * 4));
-        A(alloc_n(s, &B.srd_bhead, Cs));
+        A(alloc_n(s, &B.srd_btab, Cs * 5));  // one allocation: srd_btab, srd_bhead
+        B.srd_bhead = B.srd_btab + Cs * 4;
         A(alloc_n(s, &B.srd_bnext, nb));
         A(alloc_n(s, &B.srd_state, kSrdWords));
         A(alloc_n(s, &B.srd_start, Cs + 8));

@@ -5,9 +5,15 @@
 
 namespace nw {
 
+uint32_t bead_threads(uint64_t nb)
+{
+    return nb < 256ull * 2u * 152u ? 128u : 256u;
+}
+
 uint32_t list_filaments_per_block(uint32_t L, uint32_t nf)
 {
-    uint32_t fpb = L >= 256 ? 1u : 256u / L;
+    const uint32_t t = bead_threads((uint64_t)L * nf);
+    uint32_t fpb = L >= t ? 1u : t / L;
     if (fpb > nf && nf > 0) fpb = nf;
     return fpb ? fpb : 1u;
 }

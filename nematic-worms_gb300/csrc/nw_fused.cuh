@@ -22,7 +22,7 @@ __host__ __device__ __forceinline__ uint32_t pro_flags(const DevParams& P)
 // launch that mostly leaves at once (about 1.2 us).  At 400,000 beads they cost
 // 0.9 us more than it, so the line lies at a third of that; 100 updates of
 // 4,000 beads (three such systems at a time) take 224 us so, and 230 with the
-// launch; alone 581 and 680.  Calls of one update keep the launch.
+// launch.  Calls of one update keep the launch.
 constexpr uint32_t kInsertBeads = 131072;
 __host__ __device__ __forceinline__ bool inserts(const DevParams& P, int nsteps)
 {
@@ -47,7 +47,13 @@ __host__ __device__ __forceinline__ bool packs(const DevParams& P)
 // Tangents of the current positions as the pro part computes them.
 uint64_t launch_bead_tangents(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s);
 
-// Filaments per block of the filament-aligned kernels (about 256 threads).
+// Threads per block of the bead kernels: 256 where that gives every SM two
+// blocks, else 128, so that a small system's warps spread over
+// the SMs (their latency is what counts there): 100 updates of 4,000 beads take
+// 215 us at 128, 216 at 64 and 224 at 256, ten of 10,000 with SRD 45.8, 46.8 and
+// 44.9, 20 of 26,000 in 3D 77.9, 78.6 and 79.9.
+uint32_t bead_threads(uint64_t nb);
+// Filaments per block of the filament-aligned kernels (about bead_threads).
 uint32_t list_filaments_per_block(uint32_t L, uint32_t nf);
 
 // pro(n) with n = *step_base + off: integrate .. hash, insert into list n.

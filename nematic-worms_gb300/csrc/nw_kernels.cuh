@@ -94,7 +94,7 @@ struct StepBuffers {
     // vstate[2..4] maximum bead displacement of update n in [2 + n % 3]
     // (float bits; the bound counts from the last list build), vstate[5] the
     // largest move of positions set from the host, vstate[6] bit b set while
-    // lcount[b] holds entries of a list build
+    // lcount[b] holds entries of a list build, vstate[7] blocks done with the move
     uint32_t *nbr, *nnb, *vstate;
     uint32_t *cell_count, *cell_offset, *cell_start, *cell_end, *chunk_count;
     float4 *sorted_pos, *sorted_vel, *sorted_tan;
