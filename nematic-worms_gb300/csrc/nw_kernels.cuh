@@ -303,20 +303,7 @@ __global__ void __launch_bounds__(512) scan_cells_kernel(uint32_t* __restrict__ 
     __shared__ uint32_t s_w[16];
     __shared__ uint32_t s_base;
     const uint32_t b = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
-    uint32_t part = 0;
-    for (uint32_t k = tid; k < b; k += 512u) part += chunk_count[k];
-    part = warp_sum(part);
-    if (lane == 0) s_w[wid] = part;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t x = lane < 16u ? s_w[lane] : 0u;
-        x = warp_sum(x);
-        if (lane == 0) s_base = x;
-    }
-    __syncthreads();
-    const uint32_t base = s_base;
-    __syncthreads();
-
+    // the chunk's counts on their way while the chunks before it are summed
     const uint32_t c0 = b * kChunk + tid * 8u;
     uint32_t cnt[8];
     uint32_t tot = 0;
@@ -329,6 +316,19 @@ __global__ void __launch_bounds__(512) scan_cells_kernel(uint32_t* __restrict__ 
 #pragma unroll
         for (int k = 0; k < 8; ++k) cnt[k] = (c0 + k < ncells) ? count[c0 + k] : 0u;
     }
+    uint32_t part = 0;
+    for (uint32_t k = tid; k < b; k += 512u) part += chunk_count[k];
+    part = warp_sum(part);
+    if (lane == 0) s_w[wid] = part;
+    __syncthreads();
+    if (wid == 0) {
+        uint32_t x = lane < 16u ? s_w[lane] : 0u;
+        x = warp_sum(x);
+        if (lane == 0) s_base = x;
+    }
+    __syncthreads();
+    const uint32_t base = s_base;
+
 #pragma unroll
     for (int k = 0; k < 8; ++k) tot += cnt[k];
     const uint32_t incl = warp_incl_scan(tot);

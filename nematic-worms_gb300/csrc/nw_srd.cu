@@ -197,7 +197,7 @@ __device__ __forceinline__ void for_warp_solvent(const DevParams& P, const uint3
 
 __device__ __forceinline__ void copy16_async(float4* to, const float4* from)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
                  : "memory");
 }
 // Brings a run of global memory (16-byte aligned, a multiple of 16 bytes) into L2.
@@ -426,8 +426,9 @@ __global__ void __launch_bounds__(256) srd_scatter_kernel(const DevParams P, con
 // the shared-memory pipe at 59 %; DRAM moves 305 MB in 94 us.  More resident
 // warps spilled (9 blocks 105 us, 10 blocks 103 us), 7 blocks took 102 us;
 // batches of 3 or 8 loads along a run 99 and 100 us.  Fetching the runs' velocities and
-// positions into L2 while their hashes are looked through took 97 to 94.5 us.
-constexpr int kCollideWarps = 4;
+// positions into L2 while their hashes are looked through took 97 to 94.5 us, blocks of two
+// warps instead of four 94.2 to 92.4 (eight: 97.9), copies past L1 another 0.8.
+constexpr int kCollideWarps = 2;
 
 // Rounded products, whatever is added to them (the compiled modes round alike).
 __device__ __forceinline__ float3 scaled_rn(float f, float4 V)
@@ -465,7 +466,7 @@ struct __align__(16) CellFactors {
 enum SrdMode { kAny = 0, kRelative = 1, kLab = 2 };
 
 template <int kMode>
-__global__ void __launch_bounds__(kCollideWarps * 32, 8) srd_collide_kernel(const DevParams P, const StepBuffers S,
+__global__ void __launch_bounds__(kCollideWarps * 32, 16) srd_collide_kernel(const DevParams P, const StepBuffers S,
                                                                          uint32_t step_off, float dt_srd,
                                                                          uint32_t buf_sel)
 {
