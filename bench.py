@@ -115,8 +115,9 @@ def alg_bytes(name: str, cfg) -> float:
         "chunk_sum": 4.0 * C,
         "scatter": 16.0 * nb,
         "stable_gather": 16.0 * nb,
-        "srd_hash": 16.0 * (nb + ns) + 8.0 * (nb + ns),
-        "srd_scatter": 16.0 * (nb + ns),
+        "srd_bead_hash": 24.0 * nb,
+        "srd_hash": 16.0 * ns + 8.0 * ns,
+        "srd_scatter": 0.0,  # buckets only where the old cell order does not hold
         # bead and solvent tables in one launch each
         "srd_scan_cells": 24.0 * Cs,
         "srd_chunk_sum": 8.0 * Cs,

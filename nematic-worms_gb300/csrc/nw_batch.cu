@@ -391,9 +391,10 @@ nw_status nw_batch_create(const NwConfig* replicas, int n, nw_batch** out)
     A(balloc(b->state_allocs, &B.force, nbt));
     A(balloc(b->state_allocs, &B.force_old, nbt));
     if (b->planar) {
-        A(balloc(b->state_allocs, &B.pk[0], 3 * nbt));  // one allocation: pk[0], pk[1], pf
-        B.pk[1] = B.pk[0] + nbt;
-        B.pf = B.pk[1] + nbt;
+        // the tangents are free during a packed call: computed when they are read
+        B.pk[0] = B.tan2[0];
+        B.pk[1] = B.tan2[1];
+        A(balloc(b->state_allocs, &B.pf, nbt));
     }
     A(balloc(b->state_allocs, &B.err, 4));
     A(balloc(b->state_allocs, &B.step_base, 1));

@@ -703,6 +703,13 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
     A(alloc_n(s, &B.cell_end, C + 8));
     A(alloc_n(s, &B.chunk_count, (size_t)s->nchunks + 1));
     A(alloc_n(s, &B.sorted_pos, nb));
+    if (packs(P0)) {
+        // during a call the tangents (computed when they are read after it) and
+        // the sorted positions (between calls) are free
+        B.pk[0] = B.tan2[0];
+        B.pk[1] = B.tan2[1];
+        B.pf = B.sorted_pos;
+    }
     if (ref && !s->lists) {
         A(alloc_n(s, &B.sorted_vel, nb));
         A(alloc_n(s, &B.sorted_tan, nb));
@@ -711,11 +718,6 @@ nw_status nw_create(const NwConfig* cfg, nw_system** out)
         const size_t LC = P0.lncells > C ? P0.lncells : C;
         for (int k = 0; k < 3; ++k) A(alloc_n(s, &B.lcount[k], LC + 8));
         for (int k = 0; k < 2; ++k) A(alloc_n(s, &B.lslot[k], LC * B.cap + 8));
-    }
-    if (packs(P0)) {
-        A(alloc_n(s, &B.pk[0], 3 * nb));  // one allocation: pk[0], pk[1], pf
-        B.pk[1] = B.pk[0] + nb;
-        B.pf = B.pk[1] + nb;
     }
     if (s->vl) {
         A(alloc_n(s, &B.nbr, (size_t)P0.vl_cap * nb + 8));

@@ -76,7 +76,8 @@ struct StepBuffers {
     uint32_t* hash2[2];
     // packed bead state of planar Verlet systems between the updates of one
     // call (kPackedIn / kPackedOut, nw_fused.cuh): (x, y, v_x, v_y) of update n
-    // in pk[n & 1], (partial force x, y, previous force x, y) in pf
+    // in pk[n & 1], (partial force x, y, previous force x, y) in pf; pk is tan2
+    // (their step does not store tangents)
     float4 *pk[2], *pf;
     // in-place views of the sorted path (= pos2[0], ...)
     float4 *pos, *vel, *force, *force_old, *tangent;
