@@ -128,6 +128,7 @@ __device__ __forceinline__ bool tangent(const ObsArgs& A, uint32_t i, float3& t)
         return true;
     }
     const Pair q = two_prod(d.x, d.x) + two_prod(d.y, d.y) + two_prod(d.z, d.z);
+    if (!(q.hi > 0.f)) return false;  // a NaN beside a number, which fmaxf passes by
     // 1 / sqrt(q) = y + y / 2 (1 - q y^2), the residual from exact products
     const float y = rsqrtf(q.hi);
     const Pair y2 = two_prod(y, y);
