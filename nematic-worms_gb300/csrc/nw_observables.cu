@@ -142,17 +142,20 @@ __device__ __forceinline__ bool tangent(const ObsArgs& A, uint32_t i, float3& t)
     return true;
 }
 
-// m |v|^2 into a pair; speeds whose squares a pair does not hold go to `odd`,
-// and so do those that are not numbers (fmaxf passes a NaN beside a number by).
+// m |v|^2 into a pair; speeds and masses whose products a pair does not hold go
+// to `odd`, and so do those that are not numbers (fmaxf passes a NaN beside a
+// number by).  In these ranges a term lies between 1e-30, where its low word
+// still has 49 bits after the high word's first, and 1e31, of which 2^31 do
+// not overflow the float that sums them.
 __device__ __forceinline__ void add_kinetic(Pair& s, double& odd, float4 v, bool three)
 {
     const float vz = three ? v.z : 0.f;
     const float big = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(vz));
-    if (big > 1e-14f && big < 1e14f) {
+    if (big > 1e-14f && big < 1e14f && v.w > 0.01f && v.w < 1e3f) {
         Pair e = two_prod(v.x, v.x) + two_prod(v.y, v.y);
         if (three) e = e + two_prod(v.z, v.z);
         add(s, v.w * e);
-    } else if (!(v.x == 0.f && v.y == 0.f && vz == 0.f)) {
+    } else if (!(v.x == 0.f && v.y == 0.f && vz == 0.f && fabsf(v.w) <= 3.4028235e38f)) {
         odd += (double)v.w * ((double)v.x * v.x + (double)v.y * v.y + (three ? (double)v.z * v.z : 0.0));
     }
 }
