@@ -441,6 +441,13 @@ __device__ __forceinline__ uint32_t mod3(unsigned long long n)
     return r >= 3u ? r - 3u : r;
 }
 
+// Place of member k of a cell in the slots of all cells (a grid of up to 2^30
+// cells has more slots than 32 bits count).
+__host__ __device__ constexpr size_t list_slot(uint32_t cell, uint32_t k, uint32_t cap)
+{
+    return (size_t)cell * cap + k;
+}
+
 // Filament of a bead index (beads are stored filament by filament).
 __device__ __forceinline__ uint32_t div_L(uint32_t i, uint32_t L) { return i / L; }
 

@@ -414,8 +414,9 @@ __device__ __forceinline__ uint32_t verlet_build(const DevParams& P, const StepB
 #pragma unroll
                 for (uint32_t p = 0; p < 2u; ++p) {
                     const uint32_t u = t + p;
-                    const uint32_t at = u < m[0] ? h[0] * CAP + u : (u < m1 ? h[1] * CAP + (u - m[0]) : h[2] * CAP + (u - m1));
-                    j[p] = u < total ? __ldg(slots + at) : i;
+                    const uint32_t c = u < m[0] ? h[0] : (u < m1 ? h[1] : h[2]);
+                    const uint32_t q = u < m[0] ? u : (u < m1 ? u - m[0] : u - m1);
+                    j[p] = u < total ? __ldg(slots + list_slot(c, q, CAP)) : i;
                 }
                 float4 x[2];
 #pragma unroll
