@@ -393,19 +393,26 @@ __device__ __forceinline__ uint32_t srd_hash(const DevParams& P, float3 p, float
 
 // periodicBoundary / dampedWallBoundary / noslipWallBoundary in
 // filament_integrator's axis order (particles_kernel_impl.cuh:34-68, 99-134);
-// planar systems (D = 2) leave the z axis alone.
+// planar systems (D = 2) leave the z axis alone.  Returns whether one box
+// length did not bring the position into the box.
 template <int D = 3>
-__device__ __forceinline__ void apply_boundaries(const DevParams& P, float3& p, float3& v, float3 dr, float rad)
+__device__ __forceinline__ bool apply_boundaries(const DevParams& P, float3& p, float3& v, float3 dr, float rad)
 {
     float* pp = &p.x;
     float* vv = &v.x;
+    bool outside = false;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const float L0 = P.origin[a], L = P.box[a];
         const int b = P.bnd[a];
         if (b == NW_PERIODIC) {
-            if (pp[a] < L0) pp[a] += L;
-            else if (pp[a] > L + L0) pp[a] -= L;
+            if (pp[a] < L0) {
+                pp[a] += L;
+                outside |= pp[a] < L0;
+            } else if (pp[a] > L + L0) {
+                pp[a] -= L;
+                outside |= pp[a] > L + L0;
+            }
         } else if (b == NW_WALL) {
             if (pp[a] < L0 + rad) {
                 pp[a] = L0 + rad;
@@ -432,6 +439,7 @@ __device__ __forceinline__ void apply_boundaries(const DevParams& P, float3& p, 
             }
         }
     }
+    return outside;
 }
 
 // n mod 3: 2^32 is 1 mod 3, so the halves' remainders add.

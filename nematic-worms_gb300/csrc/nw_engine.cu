@@ -83,7 +83,8 @@ DevParams make_dev_params(const NwConfig& c, float dt)
     fast_div_params(P.L ? P.L : 1u, P.L_m, P.L_k);
     for (int a = 0; a < 3; ++a) {
         // a listed pair stays within lj_rcut + 2 skin (and a little for rounding)
-        const float reach = (c.lj_rcut + 2.0f * skin) * 1.001f + 1e-5f * c.box[a];
+        const float ulps = 1e-6f * (std::fabs(c.origin[a]) + c.box[a]);
+        const float reach = (c.lj_rcut + 2.0f * skin) * 1.001f + 1e-5f * c.box[a] + ulps;
         P.vl_lo[a] = P.bnd[a] == NW_PERIODIC ? P.origin[a] + reach : -INFINITY;
         P.vl_hi[a] = P.bnd[a] == NW_PERIODIC ? P.origin[a] + P.box[a] - reach : INFINITY;
     }

@@ -220,7 +220,8 @@ __device__ __forceinline__ float vl_bound(const StepBuffers& S, unsigned long lo
 // Whether a listed neighbour of a bead at r may lie across a periodic
 // boundary.  Warps without such a bead (97 % of them in a box of 1,400) skip
 // the minimum image of their pairs, six of about 24 instructions each; it
-// would shift by zero, so the forces are the same to the bit.
+// would shift by zero, so the forces are the same to the bit.  Every bead is
+// inside the box where a list is used (pro_part has it rebuilt otherwise).
 template <int D>
 __device__ __forceinline__ bool near_edge(const DevParams& P, float3 r)
 {
@@ -588,7 +589,9 @@ __device__ __forceinline__ void pro_part(const DevParams& P, const StepBuffers& 
         dr.y = verlet(f.y, fo.y, v.y, p.y);
         dr.z = D == 3 ? verlet(f.z, fo.z, v.z, p.z) : 0.f;
         disp2 = dotv<D>(dr, dr);
-        apply_boundaries<D>(P, p, v, dr, P.radius);
+        // a bead set from several boxes away is wrapped by one per update: while
+        // one is outside, no list holds (near_edge), and each update builds it
+        if (apply_boundaries<D>(P, p, v, dr, P.radius)) disp2 = 3.0e38f;
         nP = make_float4(p.x, p.y, p.z, P4.w);
         nV = make_float4(v.x, v.y, v.z, V4.w);
         nFo = make_float4(f.x, f.y, D == 3 ? f.z : 0.f, Fo4.w);
