@@ -328,7 +328,8 @@ __device__ __forceinline__ float3 verlet_force_planar(const DevParams& P, const 
 
 // List build: the cell scan of wca_list_force on the Verlet grid, recording
 // every non-excluded bead within lj_rcut + skin and summing the LJ force of
-// those within lj_rcut (planar systems; verlet_build the others).
+// those within lj_rcut (planar systems, and beads whose neighbours exceed the
+// list; verlet_build the others).
 template <int CAP, int D>
 __device__ __forceinline__ float3 verlet_build_force(const DevParams& P, const StepBuffers& S,
                                                      const float4* __restrict__ pos,
@@ -366,8 +367,10 @@ __device__ __forceinline__ float3 verlet_build_force(const DevParams& P, const S
 
 // The same lists in three dimensions, where 27 cells hold fewer members each:
 // every non-excluded bead within lj_rcut + skin, cell by cell in z, y, x order,
-// each cell's by ascending index; returns the list's length (S.nbr, S.nnb).  The members of a row of three cells are visited in one
-// loop, so that its lanes run as long as the longest row and not the longest
+// each cell's by ascending index; returns their number (lists and lengths in
+// S.nbr, S.nnb; a number above the lists' capacity leaves both undone).  The
+// members of a row of three cells are visited in one loop, so that its lanes
+// run as long as the longest row and not the longest
 // of each cell, and those within the radius (one in three) enter the list by
 // insertion behind the cell's first, which orders them without ordering all
 // of the cell's slots.  The forces then come from the list.  20 updates of
@@ -440,11 +443,7 @@ __device__ __forceinline__ uint32_t verlet_build(const DevParams& P, const StepB
             }
         }
     }
-    if (k > P.vl_cap) {
-        atomicOr(S.err, (uint32_t)NW_EFLAG_NEIGHBOR_OVERFLOW);
-        k = P.vl_cap;
-    }
-    S.nnb[i] = k;
+    if (k <= P.vl_cap) S.nnb[i] = k;
     return k;
 }
 
@@ -501,7 +500,13 @@ __device__ __forceinline__ float3 list_pair_force(const DevParams& P, const Step
         }
         const uint32_t own = pick2(S.hash2, cur)[i];
         if constexpr (D == 2) return verlet_build_force<CAP, D>(P, S, pos, cnt, slots, i, r, own);
-        else return verlet_force<D, true, true>(P, S, pos, i, r, verlet_build<CAP, D>(P, S, pos, cnt, slots, i, r, own));
+        else {
+            const uint32_t k = verlet_build<CAP, D>(P, S, pos, cnt, slots, i, r, own);
+            // more neighbours than the list holds: the scan that keeps the first
+            // of them in its order and takes the force of all
+            if (k > P.vl_cap) return verlet_build_force<CAP, D>(P, S, pos, cnt, slots, i, r, own);
+            return verlet_force<D, true, true>(P, S, pos, i, r, k);
+        }
     }
     return wca_list_force<CAP, D>(P, pos, cnt, slots, i, r, pick2(S.hash2, cur)[i]);
 }
