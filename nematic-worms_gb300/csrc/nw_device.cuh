@@ -456,6 +456,16 @@ __host__ __device__ constexpr size_t list_slot(uint32_t cell, uint32_t k, uint32
     return (size_t)cell * cap + k;
 }
 
+// Rank of entry k among n indices; equal ones rank by place, so that the ranks
+// are a permutation whatever the indices are.
+__host__ __device__ inline uint32_t rank_of(const uint32_t* ids, uint32_t n, uint32_t k)
+{
+    const uint32_t x = ids[k];
+    uint32_t r = 0;
+    for (uint32_t j = 0; j < n; ++j) r += ids[j] < x || (ids[j] == x && j < k);
+    return r;
+}
+
 // Filament of a bead index (beads are stored filament by filament).
 __device__ __forceinline__ uint32_t div_L(uint32_t i, uint32_t L) { return i / L; }
 

@@ -781,12 +781,7 @@ __global__ void __launch_bounds__(kBigWarps * 32) srd_collide_big_kernel(const D
         if (fits) {
             for (uint32_t k = lane; k < n; k += 32) s_in[w][k] = raw(k);
             __syncwarp();
-            for (uint32_t k = lane; k < n; k += 32) {
-                const uint32_t x = s_in[w][k];
-                uint32_t r = 0;
-                for (uint32_t j = 0; j < n; ++j) r += s_in[w][j] < x;
-                s_id[w][r] = x;
-            }
+            for (uint32_t k = lane; k < n; k += 32) s_id[w][rank_of(s_in[w], n, k)] = s_in[w][k];
             __syncwarp();
         }
         auto member = [&](uint32_t k) -> uint32_t { return fits ? s_id[w][k] : raw(k); };
