@@ -68,6 +68,7 @@ struct DevParams {
     // step by one cell)
     uint32_t sdiv_x_m, sdiv_x_k, sdiv_xy_m, sdiv_xy_k;
     float srd_per_len[3], srd_mid[3], srd_reach[3];
+    float srd_slack[3];  // cells by which rounding may move a particle between two collisions (srd_steps)
     int32_t srd_tiles_box;
     int32_t srd_flat;  // one layer, both axes periodic
 };

@@ -114,8 +114,13 @@ DevParams make_dev_params(const NwConfig& c, float dt)
         P.srd_per_len[a] = P.srd_grid[a] > 1u ? P.srd_inv_cell[a] : 0.0f;
         P.srd_mid[a] = P.origin[a] + 0.5f * P.box[a];
         P.srd_reach[a] = P.srd_grid[a] > 1u ? P.box[a] : INFINITY;
-        const double tiled = (double)P.srd_grid[a] * P.srd_cell[a];
-        if (P.srd_grid[a] > 1u && !(std::fabs(tiled - P.box[a]) <= 1e-6 * P.box[a])) P.srd_tiles_box = 0;
+        const double miss = std::fabs((double)P.srd_grid[a] * P.srd_cell[a] - P.box[a]);
+        if (P.srd_grid[a] > 1u && !(miss <= 1e-6 * P.box[a])) P.srd_tiles_box = 0;
+        // coordinates are rounded as they are stored, streamed, wrapped and
+        // shifted, a dozen times between two collisions, each time by at most
+        // 2^-24 of the largest (a box outside); three wraps miss whole cells
+        const double far = std::fabs((double)P.origin[a]) + 2.0 * P.box[a];
+        P.srd_slack[a] = (float)(1e-4 + (3.0 * miss + kSrdRound * far) * P.srd_per_len[a]);
     }
     fast_div_params(P.lgrid[0], P.ldiv_x_m, P.ldiv_x_k);
     fast_div_params(P.lgrid[0] * P.lgrid[1], P.ldiv_xy_m, P.ldiv_xy_k);

@@ -629,6 +629,7 @@ enum : uint32_t {
     kSrdWords = 24
 };
 constexpr int kSrdSteps = 4;  // cell steps per axis the ordered path takes
+constexpr float kSrdRound = 9.5367431640625e-7f;  // 2^-20, of coordinates and shifts (DevParams::srd_slack)
 
 // Tuning of the collision's two paths (overridable at compile time):
 // blocks of srd_collide_big_kernel, and the largest cell one lane of

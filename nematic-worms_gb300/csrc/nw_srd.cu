@@ -46,8 +46,9 @@ struct SrdSteps {
 // Steps between the cell of a particle at the last collision and at this
 // one.  On an axis with cells of edge a, q = (x + shift) / a lay in [X, X + 1)
 // and has changed by d = (new shift - old shift) / a and by at most `most`
-// (plus rounding, a few ulp of the box): floor(q) - X is between
-// floor(d - s) and floor(1 + d + s).  Walls clamp both cells, so there a step
+// (plus rounding, a few ulp of the largest coordinate and of the shifts, which
+// may be far larger than the box): floor(q) - X is between floor(d - s) and
+// floor(1 + d + s).  Walls clamp both cells, so there a step
 // may also be shorter, down to none.
 __device__ __forceinline__ SrdSteps srd_steps(const DevParams& P, const uint32_t (&g)[5], float3 shift)
 {
@@ -60,9 +61,10 @@ __device__ __forceinline__ SrdSteps srd_steps(const DevParams& P, const uint32_t
         w.lo[a] = 0;
         w.n[a] = 1;
         if (P.srd_grid[a] == 1u) continue;
-        const float s = most + 1e-4f + 2e-6f * (float)P.srd_grid[a];
-        const float d = (now[a] - __uint_as_float(g[a])) * P.srd_per_len[a];
-        if (!(fabsf(d) <= 8.0f)) {
+        const float was = __uint_as_float(g[a]);
+        const float d = (now[a] - was) * P.srd_per_len[a];
+        const float s = most + P.srd_slack[a] + kSrdRound * (fabsf(now[a]) + fabsf(was)) * P.srd_per_len[a];
+        if (!(fabsf(d) + s <= 8.0f)) {
             w.ordered = 0;
             continue;
         }
