@@ -231,6 +231,15 @@ __device__ __forceinline__ uint32_t step_bits(const DevParams& P, float3 dr)
                max(__float_as_uint(fabsf(dr.y) * P.srd_per_len[1]), __float_as_uint(fabsf(dr.z) * P.srd_per_len[2])));
 }
 
+// The step with what the walls move a particle by that was outside them.
+__device__ __forceinline__ float3 step_with_walls(const DevParams& P, float3 dr, float3 before, float3 after)
+{
+    const float3 back = before - after;
+    return make_float3(P.bnd[0] == NW_PERIODIC ? dr.x : fabsf(dr.x) + fabsf(back.x),
+                       P.bnd[1] == NW_PERIODIC ? dr.y : fabsf(dr.y) + fabsf(back.y),
+                       P.bnd[2] == NW_PERIODIC ? dr.z : fabsf(dr.z) + fabsf(back.z));
+}
+
 // A particle far outside the box has no bounded step.  Only a bucketed
 // collision looks: from there on particles move by a few cells at a time and
 // are wrapped, or stopped at walls.
@@ -717,9 +726,15 @@ __global__ void __launch_bounds__(kCollideWarps * 32, 16) srd_collide_kernel(con
                 float3 p = f3(P4);
                 const float3 dr = dt_srd * v;
                 p = make_float3(fmaf(dt_srd, v.x, p.x), fmaf(dt_srd, v.y, p.y), fmaf(dt_srd, v.z, p.z));
-                if constexpr (kMode == kAny) apply_boundaries(P, p, v, dr, 0.0f);
-                else wrap_periodic(P, p);
-                moved = max(moved, ordered || near_box(P, p) ? step_bits(P, dr) : kEmpty);
+                float3 step3 = dr;
+                if constexpr (kMode == kAny) {
+                    const float3 before = p;
+                    apply_boundaries(P, p, v, dr, 0.0f);
+                    step3 = step_with_walls(P, dr, before, p);
+                } else {
+                    wrap_periodic(P, p);
+                }
+                moved = max(moved, ordered || near_box(P, p) ? step_bits(P, step3) : kEmpty);
                 const uint32_t d = (any_big ? f.sorted : sorted0) + j - (f.beads & 0x7fffffffu);
                 sp_new[d] = make_float4(p.x, p.y, p.z, P4.w);
                 sv_new[d] = make_float4(v.x, v.y, v.z, V.w);
@@ -859,8 +874,9 @@ __global__ void __launch_bounds__(kBigWarps * 32) srd_collide_big_kernel(const D
                 float3 p = f3(P4);
                 const float3 dr = dt_srd * v;
                 p = make_float3(fmaf(dt_srd, v.x, p.x), fmaf(dt_srd, v.y, p.y), fmaf(dt_srd, v.z, p.z));
+                const float3 before = p;
                 apply_boundaries(P, p, v, dr, 0.0f);
-                moved = max(moved, near_box(P, p) ? step_bits(P, dr) : kEmpty);
+                moved = max(moved, near_box(P, p) ? step_bits(P, step_with_walls(P, dr, before, p)) : kEmpty);
                 const uint32_t dst = s0 + (k - nbc);
                 sp_new[dst] = make_float4(p.x, p.y, p.z, P4.w);
                 sv_new[dst] = make_float4(v.x, v.y, v.z, V.w);

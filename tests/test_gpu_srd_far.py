@@ -85,3 +85,21 @@ def test_far_shifts(far):
 def test_usual_boxes(origin):
     c, pos, vel = _system((100.0, 60.0), origin, speed=0.3)
     _compare(c, pos, vel, _shifts())
+
+
+@pytest.mark.parametrize("kind", [abi.NW_WALL, abi.NW_WALL_NO_SLIP])
+@pytest.mark.parametrize("axes", [(1,), (0, 1)])
+def test_solvent_outside_walls(axes, kind):
+    """Solvent set some cells outside the walls is put back by a step longer
+    than its streaming; with shifts of a few cells that takes it to cells other
+    than the one at the wall."""
+    c, pos, vel = _system((41.0, 37.0), (0.0, 0.0), axes, speed=0.3)
+    for a in axes:
+        c.boundary[a] = kind
+    rng = np.random.default_rng(5)
+    nb = c.n_beads
+    out = nb + rng.permutation(c.n_solvent)[: c.n_solvent // 5]
+    for a in axes:
+        far = rng.uniform(0.5, 3.0, len(out))
+        pos[out, a] = np.where(rng.random(len(out)) < 0.5, -far, c.box[a] + far)
+    _compare(c, pos, vel, [(2.3, 2.3, 0.0), (2.3, 2.3, 0.0), (2.4, 2.2, 0.0), (-2.3, -2.4, 0.0), (-2.3, -2.4, 0.0)])
