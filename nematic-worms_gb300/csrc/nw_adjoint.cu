@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/nwgb_adjoint.h"
@@ -640,12 +641,13 @@ struct Sum<float> {
     __device__ __forceinline__ double get() const { return (double)hi + (double)lo; }
 };
 
-// One adjoint update.  Triples and bonds are evaluated once each, like the
+// One adjoint update.  G: the type whose Sum gathers the gradient terms, double
+// where single-precision terms overflow its pair (backward_t).  Triples and bonds are evaluated once each, like the
 // forces above; the thread of a triple or bond also takes its share of the
 // parameter gradients for all its beads.  For 64 x 4,000 beads the kernel that
 // took every triple's dual numbers three times and every bond's terms twice
 // ran 35.6 us an update, this one 18.8 us.
-template <class T, int N, int MAXT>
+template <class T, int N, int MAXT, class G = T>
 __global__ void __launch_bounds__(MAXT) adj_step_kernel(const AdjParams<T> P, const typename Vec4<T>::type* __restrict__ r,
                                                         const uint32_t* __restrict__ nbr,
                                                         const uint32_t* __restrict__ nnb,
@@ -657,14 +659,14 @@ __global__ void __launch_bounds__(MAXT) adj_step_kernel(const AdjParams<T> P, co
                                                         double* __restrict__ gacc)
 {
     pdl_enter();
-    __shared__ Sum<T> s_g[4][MAXT + MAXT / 32];
+    __shared__ Sum<G> s_g[4][MAXT + MAXT / 32];
     // vector columns: positions, lF, bond and drive terms, second and third
     // derivative of the triples; the drives' factor
     const Columns<T> S = columns<T>();
     constexpr uint32_t kFactor = 6 * N;
     using V = Vec<T, N>;
     const Place b = place_of(P);
-    Sum<T> g[4];  // eps, k_bend, k_bond, F_act
+    Sum<G> g[4];  // eps, k_bend, k_bond, F_act
     V ri = zero<T, N>(), lfi = ri;
     if (b.on) {
         ri = ld<T, N>(r, b.i);
@@ -779,7 +781,7 @@ __global__ void __launch_bounds__(MAXT) adj_step_kernel(const AdjParams<T> P, co
     __syncthreads();
     if (threadIdx.x < 32) {
         const uint32_t q = threadIdx.x & 3u, part = (blockDim.x + 7u) / 8u, t0 = (threadIdx.x >> 2) * part;
-        Sum<T> x;
+        Sum<G> x;
         for (uint32_t t = t0; t < t0 + part && t < blockDim.x; ++t) x.add(s_g[q][t + (t >> 5)]);
         double v = x.get();
 #pragma unroll
@@ -997,6 +999,7 @@ cudaError_t allow_long_filaments()
     cudaError_t e = cudaFuncSetAttribute(adj_update_kernel<T, N, false, 1024>, attr, force);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(adj_update_kernel<T, N, true, 1024>, attr, force);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(adj_step_kernel<T, N, 1024>, attr, step);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(adj_step_kernel<T, N, 1024, double>, attr, step);
     return e;
 }
 
@@ -1057,7 +1060,13 @@ nw_status forward_t(nw_adjoint* a, const double th[4], float* pos_out, float* ve
     return NW_OK;
 }
 
-template <class T>
+template <class T, int N, class G>
+auto step_kernel(const nw_adjoint* a)
+{
+    return a->threads > 256 ? adj_step_kernel<T, N, 1024, G> : adj_step_kernel<T, N, 256, G>;
+}
+
+template <class T, class G = T>
 nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double out[4])
 {
     using V = typename Vec4<T>::type;
@@ -1078,8 +1087,7 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
         e = a->planar ? run_segment<T, 2>(a, P, (uint32_t)s, true) : run_segment<T, 3>(a, P, (uint32_t)s, true);
         const int m0 = s * a->seg + 1, m1 = std::min(a->horizon, (s + 1) * a->seg) + 1;
         for (int m = m1 - 1; m >= m0 && e == cudaSuccess; --m) {
-            auto* step = a->planar ? (a->threads > 256 ? adj_step_kernel<T, 2, 1024> : adj_step_kernel<T, 2, 256>)
-                                   : (a->threads > 256 ? adj_step_kernel<T, 3, 1024> : adj_step_kernel<T, 3, 256>);
+            auto* step = a->planar ? step_kernel<T, 2, G>(a) : step_kernel<T, 3, G>(a);
             launch_pdl(step, nbk, a->threads, (size_t)a->threads * kStepCols * sizeof(T), a->stream, P,
                        static_cast<const V*>(at(a->traj, (size_t)(m - m0), a)), a->nbr, a->nnb, static_cast<V*>(a->lr),
                        static_cast<V*>(a->lv), static_cast<const V*>(a->lF[cur]), static_cast<V*>(a->lF[cur ^ 1u]),
@@ -1104,6 +1112,10 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
         for (uint32_t b = 0; b < nbk; ++b) x += g[(size_t)b * 4 + q];
         out[q] = x;
     }
+    // a pair of floats makes NaN of an infinite term or sum: again in doubles
+    if constexpr (std::is_same_v<G, float>)
+        for (int q = 0; q < 4; ++q)
+            if (!std::isfinite(out[q])) return backward_t<T, double>(a, gpos, gvel, out);
     return NW_OK;
 }
 
