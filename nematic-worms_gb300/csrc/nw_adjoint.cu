@@ -858,7 +858,7 @@ struct nw_adjoint {
     std::vector<void*> allocs;
     double theta[4] = {0, 0, 0, 0};
     bool have_forward = false;
-    bool planar = false;  // two-dimensional, and every z of the initial state is zero: so it stays
+    bool planar = false;  // two-dimensional, every z of the initial state is zero and stays so
     float fwd_ms = 0.f, bwd_ms = 0.f;
     uint32_t lg[3] = {1, 1, 1}, lcells = 1, cap = 16, ncap = 32;
 };
@@ -1258,7 +1258,9 @@ nw_status nw_adj_set_state(nw_adjoint* a, const float* d_pos, const float* d_vel
     uint32_t out = 1;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&out, off, 4, cudaMemcpyDeviceToHost, a->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
-    a->planar = a->cfg.dim == 2 && out == 0u;
+    // z stays zero where the box holds it (else each update wraps it towards the box)
+    const float lo = a->cfg.origin[2], hi = lo + a->cfg.box[2];
+    a->planar = a->cfg.dim == 2 && out == 0u && lo <= 0.f && hi >= 0.f;
     a->have_forward = false;
     return st_of(e);
 }
