@@ -20,6 +20,7 @@
 // explicitly.  Every bead's output has one writer; per-block parameter
 // gradients are summed in a fixed order, so runs are bit-reproducible.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -792,10 +793,10 @@ __global__ void __launch_bounds__(MAXT) adj_step_kernel(const AdjParams<T> P, co
 
 // ---- conversions -------------------------------------------------------------------
 
-// xyz of a float4 array; *off_plane is set where a z component is not zero
+// xyz of a float4 array; *off_plane is set where a z component exceeds most, or is NaN
 template <class T>
 __global__ void from_f4_kernel(const float4* __restrict__ a, typename Vec4<T>::type* __restrict__ b, uint32_t n,
-                               uint32_t* __restrict__ off_plane)
+                               uint32_t* __restrict__ off_plane, float most)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const float4 q = i < n ? a[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -806,7 +807,7 @@ __global__ void from_f4_kernel(const float4* __restrict__ a, typename Vec4<T>::t
         x.c[2] = q.z;
         st(b, i, x);
     }
-    if (off_plane && __any_sync(0xffffffffu, q.z != 0.f) && (threadIdx.x & 31u) == 0u) *off_plane = 1u;
+    if (__any_sync(0xffffffffu, !(fabsf(q.z) <= most)) && (threadIdx.x & 31u) == 0u) *off_plane = 1u;
 }
 
 template <class T>
@@ -1067,7 +1068,7 @@ auto step_kernel(const nw_adjoint* a)
 }
 
 template <class T, class G = T>
-nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double out[4])
+nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double out[4], bool planar)
 {
     using V = typename Vec4<T>::type;
     const AdjParams<T> P = adj_params<T>(a, a->theta);
@@ -1077,17 +1078,20 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, a->stream);
-    from_f4_kernel<T><<<nblocks(a->N), 256, 0, a->stream>>>((const float4*)gpos, static_cast<V*>(a->lr), a->N, nullptr);
-    from_f4_kernel<T><<<nblocks(a->N), 256, 0, a->stream>>>((const float4*)gvel, static_cast<V*>(a->lv), a->N, nullptr);
-    cudaError_t e = cudaMemsetAsync(a->lF[0], 0, bytes, a->stream);
+    uint32_t* off = a->err + 1;
+    cudaError_t e = cudaMemsetAsync(off, 0, 4, a->stream);
+    for (int k = 0; k < 2; ++k)
+        from_f4_kernel<T><<<nblocks(a->N), 256, 0, a->stream>>>((const float4*)(k ? gvel : gpos),
+                                                                static_cast<V*>(k ? a->lv : a->lr), a->N, off, FLT_MAX);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a->lF[0], 0, bytes, a->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(a->lFo, 0, bytes, a->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(a->gacc, 0, (size_t)nbk * 4 * sizeof(double), a->stream);
     uint32_t cur = 0;
     for (int s = (int)a->nseg - 1; s >= 0 && e == cudaSuccess; --s) {
-        e = a->planar ? run_segment<T, 2>(a, P, (uint32_t)s, true) : run_segment<T, 3>(a, P, (uint32_t)s, true);
+        e = planar ? run_segment<T, 2>(a, P, (uint32_t)s, true) : run_segment<T, 3>(a, P, (uint32_t)s, true);
         const int m0 = s * a->seg + 1, m1 = std::min(a->horizon, (s + 1) * a->seg) + 1;
         for (int m = m1 - 1; m >= m0 && e == cudaSuccess; --m) {
-            auto* step = a->planar ? step_kernel<T, 2, G>(a) : step_kernel<T, 3, G>(a);
+            auto* step = planar ? step_kernel<T, 2, G>(a) : step_kernel<T, 3, G>(a);
             launch_pdl(step, nbk, a->threads, (size_t)a->threads * kStepCols * sizeof(T), a->stream, P,
                        static_cast<const V*>(at(a->traj, (size_t)(m - m0), a)), a->nbr, a->nnb, static_cast<V*>(a->lr),
                        static_cast<V*>(a->lv), static_cast<const V*>(a->lF[cur]), static_cast<V*>(a->lF[cur ^ 1u]),
@@ -1100,6 +1104,8 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
     std::vector<double> g((size_t)nbk * 4);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(g.data(), a->gacc, g.size() * sizeof(double), cudaMemcpyDeviceToHost, a->stream);
+    uint32_t undefined = 0;  // z gradients that are infinite or NaN reach the parameters: times 0, as NaN
+    if (e == cudaSuccess && planar) e = cudaMemcpyAsync(&undefined, off, 4, cudaMemcpyDeviceToHost, a->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
     if (e == cudaSuccess) cudaEventElapsedTime(&a->bwd_ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1107,6 +1113,7 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
     if (e != cudaSuccess) return st_of(e);
     const nw_status st = check_err(a);
     if (st != NW_OK) return st;
+    if (undefined) return backward_t<T, G>(a, gpos, gvel, out, false);
     for (int q = 0; q < 4; ++q) {
         double x = 0.0;
         for (uint32_t b = 0; b < nbk; ++b) x += g[(size_t)b * 4 + q];
@@ -1115,7 +1122,7 @@ nw_status backward_t(nw_adjoint* a, const float* gpos, const float* gvel, double
     // a pair of floats makes NaN of an infinite term or sum: again in doubles
     if constexpr (std::is_same_v<G, float>)
         for (int q = 0; q < 4; ++q)
-            if (!std::isfinite(out[q])) return backward_t<T, double>(a, gpos, gvel, out);
+            if (!std::isfinite(out[q])) return backward_t<T, double>(a, gpos, gvel, out, planar);
     return NW_OK;
 }
 
@@ -1246,11 +1253,11 @@ nw_status nw_adj_set_state(nw_adjoint* a, const float* d_pos, const float* d_vel
     uint32_t* off = a->err + 1;
     if (cudaMemsetAsync(off, 0, 4, a->stream) != cudaSuccess) return st_of(cudaGetLastError());
     if (a->prec == 64) {
-        from_f4_kernel<double><<<nbk, 256, 0, a->stream>>>((const float4*)d_pos, (double4*)a->r0, a->N, off);
-        from_f4_kernel<double><<<nbk, 256, 0, a->stream>>>((const float4*)d_vel, (double4*)a->v0, a->N, off);
+        from_f4_kernel<double><<<nbk, 256, 0, a->stream>>>((const float4*)d_pos, (double4*)a->r0, a->N, off, 0.f);
+        from_f4_kernel<double><<<nbk, 256, 0, a->stream>>>((const float4*)d_vel, (double4*)a->v0, a->N, off, 0.f);
     } else {
-        from_f4_kernel<float><<<nbk, 256, 0, a->stream>>>((const float4*)d_pos, (float4*)a->r0, a->N, off);
-        from_f4_kernel<float><<<nbk, 256, 0, a->stream>>>((const float4*)d_vel, (float4*)a->v0, a->N, off);
+        from_f4_kernel<float><<<nbk, 256, 0, a->stream>>>((const float4*)d_pos, (float4*)a->r0, a->N, off, 0.f);
+        from_f4_kernel<float><<<nbk, 256, 0, a->stream>>>((const float4*)d_vel, (float4*)a->v0, a->N, off, 0.f);
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(a->w_pos, d_pos, (size_t)a->N * 16, cudaMemcpyDeviceToDevice, a->stream);
@@ -1296,8 +1303,8 @@ nw_status nw_adj_backward(nw_adjoint* a, const float* d_grad_pos, const float* d
 {
     if (!a || !d_grad_pos || !d_grad_vel || !grad_theta) return NW_ERR_INVALID;
     if (!a->have_forward) return NW_ERR_INVALID;
-    return a->prec == 64 ? backward_t<double>(a, d_grad_pos, d_grad_vel, grad_theta)
-                         : backward_t<float>(a, d_grad_pos, d_grad_vel, grad_theta);
+    return a->prec == 64 ? backward_t<double>(a, d_grad_pos, d_grad_vel, grad_theta, a->planar)
+                         : backward_t<float>(a, d_grad_pos, d_grad_vel, grad_theta, a->planar);
 }
 
 nw_status nw_adj_timings(const nw_adjoint* a, float* forward_ms, float* backward_ms)
