@@ -18,6 +18,15 @@ uint32_t list_filaments_per_block(uint32_t L, uint32_t nf)
     return fpb ? fpb : 1u;
 }
 
+bool inserts(const DevParams& P, int nsteps)
+{
+    if (!P.vl_on || nsteps <= 1 || P.nb == 0) return false;
+    uint32_t fpb, threads;
+    size_t smem;
+    pro_shape(P, fpb, threads, smem);
+    return (uint64_t)cdiv32(P.nf, fpb) * threads <= kInsertThreads;
+}
+
 uint64_t launch_bead_pro(const DevParams& P, const StepBuffers& B, uint32_t off, float dt, uint32_t packed,
                          uint32_t insert, cudaStream_t s)
 {

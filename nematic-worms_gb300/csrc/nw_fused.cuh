@@ -19,15 +19,16 @@ __host__ __device__ __forceinline__ uint32_t pro_flags(const DevParams& P)
 }
 // Small Verlet systems fill every update's cell list in the pro part, although
 // only list builds read it: the atomics and the clearing cost less than a
-// launch that mostly leaves at once (about 1.2 us).  At 400,000 beads they cost
-// 0.9 us more than it, so the line lies at a third of that; 100 updates of
-// 4,000 beads (three such systems at a time) take 224 us so, and 230 with the
-// launch.  Calls of one update keep the launch.
-constexpr uint32_t kInsertBeads = 131072;
-__host__ __device__ __forceinline__ bool inserts(const DevParams& P, int nsteps)
-{
-    return P.vl_on && nsteps > 1 && P.nb <= kInsertBeads;
-}
+// launch that mostly leaves at once (about 1.2 us).  That holds while the
+// threads of two successive updates fit the chip together, six blocks of 256 on
+// each of 152 SMs, so that the next update's blocks wait on the chip and not
+// for it.  40 updates of planar beads, filled in the pro part / by the launch
+// (us): 60,000 264 / 274, 80,000 281 / 299, 110,000 285 / 310, 120,000 403 / 320,
+// 130,000 405 / 351; 20 in 3D: 80,000 216 / 219, 100,000 232 / 227, 130,000
+// 286 / 256; ten with SRD: 40,000 101 / 103, 100,000 134 / 131, 130,000
+// 164 / 149.  Calls of one update keep the launch.
+constexpr uint64_t kInsertThreads = 152ull * 6ull * 256ull / 2ull;
+bool inserts(const DevParams& P, int nsteps);
 
 // Within one call, the bead state of planar Verlet systems between updates is
 // packed: two float4 a bead (x, y, velocity; partial and previous force)
