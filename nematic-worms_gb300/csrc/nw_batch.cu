@@ -43,8 +43,8 @@ struct nw_batch {
     // launch layout of the current tuning
     std::vector<ReplicaSlot> slots;
     ReplicaSlot* d_slots = nullptr;
-    uint32_t* d_block_rep = nullptr;
-    uint32_t blocks = 0, threads = 0, cap = 8;
+    uint32_t *d_block_rep = nullptr, *d_list_rep = nullptr;
+    uint32_t blocks = 0, lblocks = 0, threads = 0, cap = 8;
     size_t smem = 0;
     StepBuffers B{};
     std::vector<void*> state_allocs, list_allocs;
@@ -172,7 +172,7 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
     b->threads = threads;
     b->smem = (size_t)threads * sizeof(float4) * (reverse ? 3u : 1u) + (size_t)threads * 3u * sizeof(float4);
     b->slots.assign(b->R, ReplicaSlot{});
-    std::vector<uint32_t> block_rep;
+    std::vector<uint32_t> block_rep, list_rep;
     uint64_t cells = 0, nbr_words = 0;
     b->vl = false;
     b->packed = true;
@@ -194,6 +194,9 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
         e.blk0 = (uint32_t)block_rep.size();
         e.nblk = c.num_filaments ? cdivu(c.num_filaments, fpb) : 0u;
         for (uint32_t k = 0; k < e.nblk; ++k) block_rep.push_back((uint32_t)r);
+        e.lblk0 = (uint32_t)list_rep.size();
+        e.lnblk = list_blocks(b->nb[r], threads);
+        list_rep.insert(list_rep.end(), e.lnblk, (uint32_t)r);
         cells += e.P.lncells;
         b->packed = b->packed && packs(e.P);
         if (e.P.vl_on) {
@@ -203,6 +206,7 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
     }
     if (cells >= (1ull << 32) || nbr_words >= (1ull << 40)) return NW_ERR_INVALID;
     b->blocks = (uint32_t)block_rep.size();
+    b->lblocks = (uint32_t)list_rep.size();
     nw_status st = NW_OK;
     auto A = [&](nw_status x) {
         if (st == NW_OK) st = x;
@@ -219,11 +223,14 @@ nw_status configure(nw_batch* b, const NwBatchTuning& t)
     }
     A(balloc(b->list_allocs, &b->d_slots, b->slots.size()));
     A(balloc(b->list_allocs, &b->d_block_rep, block_rep.size() + 1));
+    A(balloc(b->list_allocs, &b->d_list_rep, list_rep.size() + 1));
     if (st != NW_OK) return st;
     cudaError_t e = cudaMemcpy(b->d_slots, b->slots.data(), b->slots.size() * sizeof(ReplicaSlot),
                                cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !block_rep.empty())
         e = cudaMemcpy(b->d_block_rep, block_rep.data(), block_rep.size() * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !list_rep.empty())
+        e = cudaMemcpy(b->d_list_rep, list_rep.data(), list_rep.size() * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_st(e);
     b->tune = t;
     b->tune.cell_capacity = b->cap;
@@ -264,9 +271,9 @@ uint64_t enqueue(nw_batch* b, int nsteps)
     if (b->blocks == 0) return 0;
     uint64_t launches = 0;
     auto L = [&](int mode, uint32_t off, uint32_t packed) {
-        const uint32_t blocks = mode == kBatchList ? (uint32_t)b->R * kBatchListBlocks : b->blocks;
-        launch_batch(mode, b->d_slots, b->d_block_rep, blocks, b->threads, b->smem, b->cap, b->B, off, b->planar,
-                     packed, b->stream);
+        const bool list = mode == kBatchList;
+        launch_batch(mode, b->d_slots, list ? b->d_list_rep : b->d_block_rep, list ? b->lblocks : b->blocks,
+                     b->threads, b->smem, b->cap, b->B, off, b->planar, packed, b->stream);
         ++launches;
     };
     // every update but the last leaves its state packed

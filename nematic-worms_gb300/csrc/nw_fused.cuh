@@ -87,16 +87,29 @@ struct ReplicaSlot {
     uint32_t blk0;      // first block of the launch
     uint32_t nblk;      // blocks of this replica
     uint32_t fpb;       // filaments per block
-    uint32_t pad[2];
+    uint32_t lblk0, lnblk;  // the same of the list launch (list_blocks of the replica's beads)
     unsigned long long nbr_off;  // first neighbour-list word
 };
 
 // kBatchList: a replica's cell list of update n when its pair pass will
-// rebuild the Verlet lists (Verlet replicas; launched after each pro part);
-// kBatchListBlocks blocks for each replica, which mostly leave at once
-constexpr uint32_t kBatchListBlocks = 8;
+// rebuild the Verlet lists (Verlet replicas; launched after each pro part), by
+// list_blocks blocks of a replica, which mostly leave at once
 enum BatchMode { kBatchPro = 0, kBatchEpi = 1, kBatchFused = 2, kBatchList = 3 };
 
+// Blocks that build one replica's cell list: up to eight, and eight beads a
+// thread, four of them in flight, from 16,384 beads (of 256 threads) on.  The
+// launch costs with its blocks where no replica rebuilds, a rebuild with the
+// beads of a thread.  20 updates of replicas x beads, eight blocks each whatever
+// the size / this rule / a thread a bead, us: 1 x 400,000 549 / 350 / 390,
+// 16 x 100,000 1,803 / 1,301 / 1,540, 8 x 60,000 630 / 483 / 513, 64 x 60,000
+// 3,555 / 3,049 / 3,541, 64 x 20,000 1,261 / 1,187 / 1,386, 64 x 4,000
+// 471 / 473 / 489; 16 beads a thread 8 x 60,000 517, four 466, but 64 uneven
+// replicas of 250 to 60,000 beads 1,057 instead of 1,038 (1,031 with eight blocks).
+inline uint32_t list_blocks(uint32_t beads, uint32_t threads)
+{
+    const uint32_t one = (beads + threads - 1u) / threads, eight = (one + 7u) / 8u;  // blocks for one and eight beads a thread
+    return eight > 8u ? eight : one < 8u ? one : 8u;
+}
 // One launch over all replicas: block b serves replica block_rep[b].  S holds
 // the batch's base pointers; `threads` >= every replica's fpb * L; planar =
 // every replica is a planar system.

@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
 {
     pdl_enter();
     __shared__ DevParams sP;
-    const uint32_t r = MODE == kBatchList ? blockIdx.x / kBatchListBlocks : __ldg(block_rep + blockIdx.x);
+    const uint32_t r = __ldg(block_rep + blockIdx.x);
     const ReplicaSlot* e = table + r;
     if (MODE == kBatchList) {
         // leave before staging the parameter block unless this replica rebuilds
@@ -847,13 +847,24 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? 6 : 1) batch_kernel(const 
         // this replica's cell list of update n, only when its pair pass rebuilds
         const uint32_t out = (uint32_t)(n & 1ull);
         const float4* __restrict__ pos = kPacked ? pick2(S.pk, out) : pick2(S.pos2, out);
-        for (uint32_t j = (blockIdx.x % kBatchListBlocks) * blockDim.x + threadIdx.x; j < P.nb;
-             j += kBatchListBlocks * blockDim.x) {
-            const uint32_t h = list_hash(P, f3(pos[j]));
-            pick2(S.hash2, out)[j] = h;
-            const uint32_t slot = atomicAdd(&pick3(S.lcount, mod3(n))[h], 1u);
-            if (slot < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h * CAP + slot] = j;
-            else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
+        // four beads of a thread in flight
+        const uint32_t stride = e->lnblk * blockDim.x;
+        uint32_t* cnt = pick3(S.lcount, mod3(n));
+        for (uint32_t j0 = (blockIdx.x - e->lblk0) * blockDim.x + threadIdx.x; j0 < P.nb; j0 += 4u * stride) {
+            uint32_t h[4], slot[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; ++q) h[q] = j0 + q * stride < P.nb ? list_hash(P, f3(pos[j0 + q * stride])) : kEmpty;
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; ++q)
+                if (h[q] != kEmpty) slot[q] = atomicAdd(cnt + h[q], 1u);
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; ++q) {
+                if (h[q] == kEmpty) continue;
+                const uint32_t j = j0 + q * stride;
+                pick2(S.hash2, out)[j] = h[q];
+                if (slot[q] < (uint32_t)CAP) pick2(S.lslot, out)[(size_t)h[q] * CAP + slot[q]] = j;
+                else atomicOr(S.err, (uint32_t)NW_EFLAG_CELL_OVERFLOW);
+            }
         }
         return;
     }
