@@ -294,6 +294,9 @@ nw_status nw_set_stream(nw_system* sys, void* stream);
 nw_status nw_set_graphs(nw_system* sys, int enabled);
 /* Run only the SRD sub-step (for tests): shift given in world units. */
 nw_status nw_srd_collide(nw_system* sys, float dt_srd, const float shift[3]);
+/* Whether the last collision found its solvent through the stored cell order
+ * (1) or bucketed it (0); both give the same results (for tests). */
+nw_status nw_srd_ordered(nw_system* sys, int* ordered);
 
 /* ---- checkpoint / resume -------------------------------------------------- */
 

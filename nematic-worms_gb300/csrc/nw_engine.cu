@@ -1104,6 +1104,17 @@ nw_status nw_srd_collide(nw_system* s, float dt_srd, const float shift[3])
     return cuda_status(e);
 }
 
+nw_status nw_srd_ordered(nw_system* s, int* ordered)
+{
+    if (!s || !ordered) return NW_ERR_INVALID;
+    if (!s->B.srd_state) return NW_ERR_UNSUPPORTED;
+    uint32_t w = 0;
+    cudaError_t e = cudaMemcpyAsync(&w, s->B.srd_state + kSrdOrdered, 4, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    *ordered = (int)w;
+    return cuda_status(e);
+}
+
 // ---- checkpoints ---------------------------------------------------------------
 
 struct CkptHeader {

@@ -223,6 +223,7 @@ HANDLE_API = [
     ("nw_set_stream", C.c_int, [_sysp, _P]),
     ("nw_set_graphs", C.c_int, [_sysp, C.c_int]),
     ("nw_srd_collide", C.c_int, [_sysp, _f32, C.POINTER(_f32)]),
+    ("nw_srd_ordered", C.c_int, [_sysp, C.POINTER(C.c_int)]),
     ("nw_checkpoint_size", C.c_int, [_sysp, C.POINTER(C.c_size_t)]),
     ("nw_checkpoint_save", C.c_int, [_sysp, _P, C.c_size_t]),
     ("nw_checkpoint_load", C.c_int, [_sysp, _P, C.c_size_t]),

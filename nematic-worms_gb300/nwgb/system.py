@@ -161,6 +161,14 @@ class System:
         check(self.lib.nw_srd_collide(self._h, float(dt_srd), s), "nw_srd_collide")
 
     @property
+    def srd_ordered(self) -> bool:
+        """Whether the last collision found its solvent through the stored
+        cell order (else it bucketed it; the results are the same)."""
+        n = C.c_int()
+        check(self.lib.nw_srd_ordered(self._h, C.byref(n)), "nw_srd_ordered")
+        return bool(n.value)
+
+    @property
     def last_launch_count(self) -> int:
         n = C.c_uint64()
         check(self.lib.nw_last_launch_count(self._h, C.byref(n)))
