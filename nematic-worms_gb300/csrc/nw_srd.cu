@@ -231,13 +231,12 @@ __device__ __forceinline__ uint32_t step_bits(const DevParams& P, float3 dr)
                max(__float_as_uint(fabsf(dr.y) * P.srd_per_len[1]), __float_as_uint(fabsf(dr.z) * P.srd_per_len[2])));
 }
 
-// The step with what the walls move a particle by that was outside them.
-__device__ __forceinline__ float3 step_with_walls(const DevParams& P, float3 dr, float3 before, float3 after)
+// A particle's way from `was`: its streaming step on periodic axes; on the
+// others also what a wall put it back by where it was outside.
+__device__ __forceinline__ float3 way_of(const DevParams& P, float3 dr, float4 was, float3 now)
 {
-    const float3 back = before - after;
-    return make_float3(P.bnd[0] == NW_PERIODIC ? dr.x : fabsf(dr.x) + fabsf(back.x),
-                       P.bnd[1] == NW_PERIODIC ? dr.y : fabsf(dr.y) + fabsf(back.y),
-                       P.bnd[2] == NW_PERIODIC ? dr.z : fabsf(dr.z) + fabsf(back.z));
+    return make_float3(P.bnd[0] == NW_PERIODIC ? dr.x : now.x - was.x, P.bnd[1] == NW_PERIODIC ? dr.y : now.y - was.y,
+                       P.bnd[2] == NW_PERIODIC ? dr.z : now.z - was.z);
 }
 
 // A particle far outside the box has no bounded step.  Only a bucketed
@@ -726,15 +725,10 @@ __global__ void __launch_bounds__(kCollideWarps * 32, 16) srd_collide_kernel(con
                 float3 p = f3(P4);
                 const float3 dr = dt_srd * v;
                 p = make_float3(fmaf(dt_srd, v.x, p.x), fmaf(dt_srd, v.y, p.y), fmaf(dt_srd, v.z, p.z));
-                float3 step3 = dr;
-                if constexpr (kMode == kAny) {
-                    const float3 before = p;
-                    apply_boundaries(P, p, v, dr, 0.0f);
-                    step3 = step_with_walls(P, dr, before, p);
-                } else {
-                    wrap_periodic(P, p);
-                }
-                moved = max(moved, ordered || near_box(P, p) ? step_bits(P, step3) : kEmpty);
+                if constexpr (kMode == kAny) apply_boundaries(P, p, v, dr, 0.0f);
+                else wrap_periodic(P, p);
+                const float3 way = kMode == kAny ? way_of(P, dr, P4, p) : dr;
+                moved = max(moved, ordered || near_box(P, p) ? step_bits(P, way) : kEmpty);
                 const uint32_t d = (any_big ? f.sorted : sorted0) + j - (f.beads & 0x7fffffffu);
                 sp_new[d] = make_float4(p.x, p.y, p.z, P4.w);
                 sv_new[d] = make_float4(v.x, v.y, v.z, V.w);
@@ -798,7 +792,17 @@ __global__ void __launch_bounds__(kBigWarps * 32) srd_collide_big_kernel(const D
         if (fits) {
             for (uint32_t k = lane; k < n; k += 32) s_in[w][k] = raw(k);
             __syncwarp();
-            for (uint32_t k = lane; k < n; k += 32) s_id[w][rank_of(s_in[w], n, k)] = s_in[w][k];
+            uint32_t ranks = 0;
+            for (uint32_t k = lane; k < n; k += 32) {
+                const uint32_t x = s_in[w][k];
+                uint32_t r = 0;
+                for (const uint32_t* y = s_in[w]; y < s_in[w] + n; ++y) r += *y < x;
+                s_id[w][r] = x;
+                ranks += r;
+            }
+            // ranks of indices that repeat fall short: they would leave places unwritten
+            if (__reduce_add_sync(0xffffffffu, ranks) != n * (n - 1u) / 2u)
+                for (uint32_t k = lane; k < n; k += 32) s_id[w][rank_of(s_in[w], n, k)] = s_in[w][k];
             __syncwarp();
         }
         auto member = [&](uint32_t k) -> uint32_t { return fits ? s_id[w][k] : raw(k); };
@@ -874,9 +878,8 @@ __global__ void __launch_bounds__(kBigWarps * 32) srd_collide_big_kernel(const D
                 float3 p = f3(P4);
                 const float3 dr = dt_srd * v;
                 p = make_float3(fmaf(dt_srd, v.x, p.x), fmaf(dt_srd, v.y, p.y), fmaf(dt_srd, v.z, p.z));
-                const float3 before = p;
                 apply_boundaries(P, p, v, dr, 0.0f);
-                moved = max(moved, near_box(P, p) ? step_bits(P, step_with_walls(P, dr, before, p)) : kEmpty);
+                moved = max(moved, near_box(P, p) ? step_bits(P, way_of(P, dr, P4, p)) : kEmpty);
                 const uint32_t dst = s0 + (k - nbc);
                 sp_new[dst] = make_float4(p.x, p.y, p.z, P4.w);
                 sv_new[dst] = make_float4(v.x, v.y, v.z, V.w);
