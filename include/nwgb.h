@@ -411,7 +411,8 @@ nw_status nw_sample_defects(nw_system* sys, const uint32_t* beads, int n_points,
  *    nw_observe_reset, unwrapped by the periodic images each bead crossed
  *    between calls (call at least once per half box of motion; bead indices
  *    must not move, so no filament reversal in between).
- * Fixed-order double sums.  Synchronous. */
+ * Fixed-order sums of pairs of floats and doubles, within 1e-13 of double
+ * sums.  Synchronous. */
 #define NW_OBS_MIN_IMAGE 1u
 #define NW_OBS_MSD 2u
 typedef struct NwObservables {

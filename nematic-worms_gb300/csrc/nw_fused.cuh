@@ -49,10 +49,12 @@ __host__ __device__ __forceinline__ bool packs(const DevParams& P)
 uint64_t launch_bead_tangents(const DevParams& P, const float4* pos, float4* tan, cudaStream_t s);
 
 // Threads per block of the bead kernels: 256 where that gives every SM two
-// blocks, else 128, so that a small system's warps spread over
-// the SMs (their latency is what counts there): 100 updates of 4,000 beads take
-// 215 us at 128, 216 at 64 and 224 at 256, ten of 10,000 with SRD 45.8, 46.8 and
-// 44.9, 20 of 26,000 in 3D 77.9, 78.6 and 79.9.
+// blocks, else 128, so that a small system's warps spread over the SMs (their
+// latency is what counts there).  128 / 256, us: 40 updates of planar beads
+// 4,000 210 / 220, 40,000 238 / 245, 77,000 260 / 269, 160,000 350 / 358, 300,000
+// 527 / 517; 20 in 3D: 26,000 176 / 181, 50,000 186 / 192, 77,000 203 / 198,
+// 120,000 283 / 283; ten with SRD: 10,000 83.5 / 84.4, 25,000 90.3 / 89.6, 50,000
+// 95.2 / 96.1, 77,000 112 / 111 (several systems of 10,000 in turn 45.8 / 44.9).
 uint32_t bead_threads(uint64_t nb);
 // Filaments per block of the filament-aligned kernels (about bead_threads).
 uint32_t list_filaments_per_block(uint32_t L, uint32_t nf);

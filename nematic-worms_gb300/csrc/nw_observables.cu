@@ -4,10 +4,11 @@
 // velocity correlation of sampled bead pairs by distance, and the histogram
 // of SRD cell temperatures.
 //
-// Sums are deterministic: per-block partial sums in double, reduced by one
-// block in block order (nw_observe, nw_velocity_correlation), or integer
-// atomics on fixed-point values (the SRD cell sums: the same integers
-// whatever the thread order).
+// Sums are deterministic: a thread's and a warp's as unevaluated pairs of
+// floats (nw_observe; doubles in nw_velocity_correlation), a block's in
+// doubles, and the blocks' partial sums by one block, a warp per sum, in a
+// fixed order; or integer atomics on fixed-point values (the SRD cell sums: the
+// same integers whatever the thread order).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

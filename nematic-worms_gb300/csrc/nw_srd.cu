@@ -432,12 +432,13 @@ __global__ void __launch_bounds__(256) srd_scatter_kernel(const DevParams P, con
 //
 // What bounds it: 61M warp instructions (of 1,900 a warp some 400 find the
 // members, 500 are the two serial sums over a cell, whose longest of 32 has 10
-// members for 4.4 on average, 500 the update) at 53 % of the issue rate, and
-// the shared-memory pipe at 59 %; DRAM moves 305 MB in 94 us.  More resident
-// warps spilled (9 blocks 105 us, 10 blocks 103 us), 7 blocks took 102 us;
-// batches of 3 or 8 loads along a run 99 and 100 us.  Fetching the runs' velocities and
-// positions into L2 while their hashes are looked through took 97 to 94.5 us, blocks of two
-// warps instead of four 94.2 to 92.4 (eight: 97.9), copies past L1 another 0.8.
+// members for 4.4 on average, 500 the update) at 58 % of the issue rate, and
+// the shared-memory pipe at 56 %; DRAM moves 306 MB in 92 us.  With blocks of
+// four warps, 8 of them resident, more warps spilled (9 blocks 105 us, 10
+// blocks 103 us) and fewer (7 blocks) took 102 us; batches of 3 or 8 loads along
+// a run 99 and 100 us.  Fetching the runs' velocities and positions into L2 while
+// their hashes are looked through took 97 to 94.5 us, blocks of two warps (16
+// resident) instead of four 94.2 to 92.4 (eight: 97.9), copies past L1 another 0.8.
 constexpr int kCollideWarps = 2;
 
 // Rounded products, whatever is added to them (the compiled modes round alike).
