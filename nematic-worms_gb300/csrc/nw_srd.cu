@@ -931,15 +931,18 @@ uint64_t enqueue_srd(const DevParams& P, const StepBuffers& B, uint32_t srd_nchu
     NW_MARK("srd_collide_big");
     // Few cells of a fresh dilute solvent are big, but many of a late state,
     // crowded at walls or by the beads: a block for 1,024 cells and at least one
-    // an SM; in a dense solvent for 256 cells and at least two an SM.  Calls of ten
-    // updates, after 200 of them / 50,000, us, with a block for 1,024 cells alone,
-    // so, and with 912 blocks: 5,460 beads between walls 61.1 / 95.7,
-    // 61.5 / 80.1, 64.9 / 83.0; 4,335 between walls 49.0 / 89.0, 49.2 / 67.1,
-    // 51.2 / 70.6; 22,056 58.0 / 84.2, 58.6 / 76.4, 63.1 / 80.5.  Dense, five updates
-    // after 100 / 12,500, with a block for four cells (up to 912) and with 304: 4,800
-    // REF_DEM beads on 64 x 64 solvent cells 86.5 / 97, 78.3 / 89.5; 72,000 on
-    // 256 x 256 153 / 163, 142 / 153; 180,000 on 512 x 512 331 / 342, 326 / 346.
-    const uint32_t big_blocks = dense ? std::max(304u, cdiv(P.srd_ncells, 256)) : std::max(152u, cdiv(P.srd_ncells, 1024));
+    // an SM, two between walls; in a dense solvent for 256 cells and at least two
+    // an SM.  Calls of ten updates, after 200 of them / 60,000, us, with a block for
+    // 1,024 cells alone, with 152 blocks at least, 304, and 912 always: 22,056 beads
+    // 58.0 / 84.2, 58.6 / 76.4, 59.2 / 75.2, 63.1 / 80.5; 5,460 between walls
+    // 61.4 / 99, 61.8 / 79.0, 62.3 / 77.5, 64.9 / 83; 11,925 between walls 83.4 / 140,
+    // 84.0 / 121, 84.4 / 114.5, late 118 with 912; 30,000 between walls 68.0 / 130,
+    // 68.7 / 123, 69.3 / 108.6, late 109.  Dense, five updates after 100 / 12,500,
+    // with a block for four cells (up to 912) and with 304: 4,800 REF_DEM beads on
+    // 64 x 64 solvent cells 86.5 / 97, 78.3 / 89.5; 72,000 on 256 x 256 153 / 163,
+    // 142 / 153; 180,000 on 512 x 512 331 / 342, 326 / 346.
+    const uint32_t big_blocks =
+        std::max(dense || !periodic ? 304u : 152u, cdiv(P.srd_ncells, dense ? 256u : 1024u));
     launch_pdl(srd_collide_big_kernel, std::min(kSrdBigBlocks, big_blocks), kBigWarps * 32, 0, s, P, B, step_off,
                dt_srd, buf_sel);
     return 7;
